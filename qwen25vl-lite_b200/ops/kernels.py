@@ -64,7 +64,7 @@ _SIGNATURES = {
 _UNTYPED = {
     "q25_attention_decode_bf16": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "q25_attention_prefill_bf16": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P],
-    "q25_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    "q25_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "q25_gemm_tcgen05_bf16": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "q25_sample_rows": [_P, _LL, _I, _I, _P, _P, _P, _P, _P, _P],
     "q25_apply_penalties": [_P, _LL, _I, _I, _P, _P, _P, _P, _P, _P, _P],
@@ -438,7 +438,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
             raise KernelError(f"gemm_f32 {what}: needs a float32 CUDA matrix with unit inner stride")
     _check(_fn("q25_gemm_f32", _UNTYPED["q25_gemm_f32"])(
         a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), m, n, k, a.stride(0), w.stride(0), out.stride(0),
-        _stream()), "gemm_f32")
+        error_flag(out.device).data_ptr(), _stream()), "gemm_f32")
 
 
 SKINNY_STORE, SKINNY_BIAS, SKINNY_F32, SKINNY_SWIGLU, SKINNY_RESIDUAL, SKINNY_GLU, SKINNY_RELU2, SKINNY_RESIDUAL_SCALED = 0, 1, 2, 3, 4, 5, 6, 7
