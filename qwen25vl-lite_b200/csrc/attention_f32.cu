@@ -1,0 +1,521 @@
+// Causal attention over the paged cache in true 32-bit, heads of up to 128 channels: the attention of the 32-bit path.
+// Formula as in attention_generic.cu (reference src/qwen25vl_lite/text.py:78,156-175), which keeps the sizes this one
+// does not take.
+//
+// The keys are cut into ranges of 128, aligned to the absolute key index.  Inside a range: the scores (a dot product is two
+// chains, over the even and the odd channels), their maximum, p = exp(s - maximum), the sum of p (keys lane + 32 j by lane,
+// then a butterfly) and for every channel one chain of p v over the keys in order.  The ranges' (maximum, sum, values) are
+// then added up in order.  Nothing of this depends on how the tokens were cut into steps or on what else is in the batch, so
+// both kernels here give a query the same bits:
+//
+//   * af32_tile_kernel: runs of tokens.  A CTA takes 64 rows (token, head of the kv group), token-major, of one entry, a
+//     warp 16 of them; keys and values come in tiles of 32 through two buffers (cp.async), and both products are packed
+//     FMAs on registers (16 rows x 32 keys, then 16 rows x all channels for a warp);
+//   * af32_single_kernel: entries of one token.  A CTA takes one range of one kv head: a thread owns a key for the scores and a
+//     channel for the values; the CTA that finishes an entry's last range adds them all up.
+//
+// One warp per (token, head) on the CUDA cores with a key per lane, as before, read every key again for every row: 9.6 ms for
+// a prompt of 1,500 tokens with 16 heads of 128 (0.96 TFLOP/s), 750 us for one token at 1,500 keys.
+#include "common.cuh"
+
+#define AF_RANGE 128                             // keys of one range
+#define AF_KEYS 32                               // keys of one tile
+#define AF_ROWS 64                               // rows of a CTA of the tile kernel
+#define AF_THREADS 128
+#define AF_SPITCH 136                            // floats between rows of scores: four rows' stores lie in different banks
+#define AF_HEADS 8                               // rows the single kernel works on at a time
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 af_fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 af_pair(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 af_split(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ ulonglong2 af_lds2(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ void af_copy16(float* dst, const float* src, bool valid) {
+  const int n = valid ? 16 : 0;                  // not valid: zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void af_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+struct Af32Args {
+  const float* qkv;
+  float* out;
+  const float *kpages, *vpages;
+  const int *table, *cu_q, *start;
+  int qkv_stride, table_width, entries, nq, nkv, d, page_size, window;
+  float scale;
+  int min_run;                                   // tokens from which on an entry is the tile kernel's
+  int ranges;                                    // most ranges an entry can have (single kernel)
+  float* scratch;                                // [entry][kv head][range][head of the group][d + 2]
+  int* counters;                                 // one per (entry, kv head), zero before the launch and after it
+};
+
+// (m, l, a) of a range joins the total of the ranges before it.
+__device__ __forceinline__ void af_weights(float& m, float& l, float rm, float rl, float& c1, float& c2) {
+  const float top = fmaxf(m, rm);
+  c1 = expf(m - top);                            // the first range: exp(-inf) = 0
+  c2 = expf(rm - top);
+  l = fmaf(l, c1, rl * c2);
+  m = top;
+}
+
+// ---- runs of tokens ---------------------------------------------------------------------------------------------------
+// NJ: runs of 32 channels, the head's channels rounded up.
+template <int NJ>
+__global__ void __launch_bounds__(AF_THREADS, 2) af32_tile_kernel(const Af32Args A) {
+  extern __shared__ __align__(16) float af_smem[];
+  const int d = A.d, pitch = d + 4, g = A.nq / A.nkv;           // rows of an odd number of 16-byte chunks: no bank conflicts
+  float* qs = af_smem;
+  float* ss = qs + AF_ROWS * pitch;
+  float* ring = ss + AF_ROWS * AF_SPITCH;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = lane & 7, ty = lane >> 3;
+  const int kvh = blockIdx.y;
+  __shared__ int place[2];
+  pdl_trigger();
+  // which entry's which tile this CTA has: entries that are the other kernel's have none (the lists come with the step's copy)
+  if (warp == 0) {
+    int before = 0, entry = -1, tile = 0;
+    for (int e0 = 0; e0 < A.entries && entry < 0; e0 += 32) {
+      const int e = e0 + lane;
+      const int q = e < A.entries ? A.cu_q[e + 1] - A.cu_q[e] : 0;
+      const int tiles = q >= A.min_run ? (q * g + AF_ROWS - 1) / AF_ROWS : 0;
+      int sum = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+      }
+      const int first = before + sum - tiles;
+      const unsigned hit = __ballot_sync(0xffffffffu, (int)blockIdx.x >= first && (int)blockIdx.x < first + tiles);
+      if (hit) {
+        const int src = __ffs(hit) - 1;
+        entry = e0 + src;
+        tile = (int)blockIdx.x - __shfl_sync(0xffffffffu, first, src);
+      }
+      before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) { place[0] = entry; place[1] = tile; }
+  }
+  __syncthreads();
+  const int entry = place[0];
+  pdl_wait();
+  if (entry < 0) return;
+  // the tiles at the end of a run see the most keys and begin first
+  const int tok0 = A.cu_q[entry], q_len = A.cu_q[entry + 1] - tok0, start = A.start[entry];
+  const int n_rows = q_len * g, row0 = ((n_rows + AF_ROWS - 1) / AF_ROWS - 1 - place[1]) * AF_ROWS;
+  const int* table = A.table + (size_t)entry * A.table_width;
+  const int chunks = d >> 2;
+
+  for (int i = tid; i < AF_ROWS * chunks; i += AF_THREADS) {
+    const int r = i / chunks, c = i - r * chunks, row = row0 + r;
+    const int token = row / g, head = kvh * g + row - token * g;
+    af_copy16(qs + r * pitch + c * 4, A.qkv + (size_t)(tok0 + (row < n_rows ? token : 0)) * A.qkv_stride + (size_t)(row < n_rows ? head : 0) * d + c * 4,
+              row < n_rows);
+  }
+  const int last_row = min(row0 + AF_ROWS, n_rows) - 1;
+  const int key_hi = start + last_row / g;                                        // last key any row sees
+  const int key_lo = A.window > 0 ? max(0, start + row0 / g - A.window + 1) : 0;  // first key any row sees
+  const int key_all = start + row0 / g;                                           // keys up to here every row sees, if no window hides them
+  const int key_clear = A.window > 0 ? max(0, key_hi - A.window + 1) : 0;         // keys from here on no window hides
+  // this warp's rows in the value product and the scores: warp * 16 + ty + 4 i
+  int pos[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) pos[i] = start + min(row0 + warp * 16 + ty + 4 * i, n_rows - 1) / g;
+
+  // the tiles of 32 keys in the order they are read: a range's keys, then the same tiles' values
+  const int r_first = key_lo / AF_RANGE, r_last = key_hi / AF_RANGE;
+  auto fetch = [&](int range, int t, bool values, int buf) {
+    float* dst = ring + buf * (AF_KEYS * pitch);
+    const float* pages = values ? A.vpages : A.kpages;
+    // lane l finds where key l lies; a copy asks the lane of its key (one look into the table a thread, not one a copy)
+    const int key0 = range * AF_RANGE + t * AF_KEYS, at = min(max(key0 + lane, key_lo), key_hi);
+    const unsigned long long off = (((unsigned long long)table[at / A.page_size] * A.nkv + kvh) * A.page_size + at % A.page_size) * d;
+    for (int i = tid; i < AF_KEYS * chunks; i += AF_THREADS) {                    // as many turns for every thread: d is a multiple of 16
+      const int k = i / chunks, c = i - k * chunks;
+      const bool valid = key0 + k >= key_lo && key0 + k <= key_hi;
+      af_copy16(dst + k * pitch + c * 4, pages + __shfl_sync(0xffffffffu, off, k) + c * 4, valid);
+    }
+    af_commit();
+  };
+  auto tiles_of = [&](int range) { return min(AF_RANGE / AF_KEYS, (key_hi - range * AF_RANGE) / AF_KEYS + 1); };
+
+  float m[4], l[4];
+  f32x2 total[4][NJ * 2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < NJ * 2; ++j) total[i][j] = 0;
+  }
+  fetch(r_first, 0, false, 0);
+  int buf = 0;
+  for (int range = r_first; range <= r_last; ++range) {
+    const int nt = tiles_of(range), base = range * AF_RANGE;
+    // ---- scores of the range ----
+    for (int t = 0; t < nt; ++t) {
+      af_wait<0>();
+      __syncthreads();
+      if (t + 1 < nt) fetch(range, t + 1, false, buf ^ 1);
+      else fetch(range, 0, true, buf ^ 1);
+      const float* ks = ring + buf * (AF_KEYS * pitch) + tx * pitch;
+      const float* qr = qs + (warp * 16 + ty) * pitch;
+      f32x2 s[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = 0;
+#pragma unroll 4
+      for (int c = 0; c < chunks; ++c) {
+        ulonglong2 q[4], k[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = af_lds2(qr + i * 4 * pitch + c * 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) k[j] = af_lds2(ks + j * 8 * pitch + c * 4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[i][j] = af_fma2(q[i].x, k[j].x, s[i][j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[i][j] = af_fma2(q[i].y, k[j].y, s[i][j]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int k = t * AF_KEYS + tx + 8 * j, key = base + k;
+          const bool seen = key <= pos[i] && (A.window <= 0 || key > pos[i] - A.window);
+          const float2 v = af_split(s[i][j]);
+          ss[(warp * 16 + ty + 4 * i) * AF_SPITCH + k] = seen ? (v.x + v.y) * A.scale : -INFINITY;
+        }
+      buf ^= 1;
+    }
+    __syncwarp();
+    // ---- probabilities, in place; this lane's rows keep their range's maximum and sum ----
+    float rm[4], rl[4];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      float* row = ss + (warp * 16 + r) * AF_SPITCH;
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = j < nt ? row[lane + 32 * j] : -INFINITY;
+      const float top = warp_max(fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])));
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = v[j] == -INFINITY ? 0.f : expf(v[j] - top);
+        if (j < nt) row[lane + 32 * j] = p;
+        sum += p;
+      }
+      sum = warp_sum(sum);
+      if ((r & 3) == ty) { rm[r >> 2] = top; rl[r >> 2] = sum; }
+    }
+    __syncwarp();
+    // ---- values ----
+    f32x2 a[4][NJ * 2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ * 2; ++j) a[i][j] = 0;
+    for (int t = 0; t < nt; ++t) {
+      af_wait<0>();
+      __syncthreads();
+      if (t + 1 < nt) fetch(range, t + 1, true, buf ^ 1);
+      else if (range < r_last) fetch(range + 1, 0, false, buf ^ 1);
+      const float* vs = ring + buf * (AF_KEYS * pitch) + tx * 4;
+      const float* pr = ss + (warp * 16 + ty) * AF_SPITCH + t * AF_KEYS;
+      const int k0 = base + t * AF_KEYS;
+      const bool every = k0 + AF_KEYS - 1 <= key_all && k0 >= key_clear;      // no row of this CTA hides a key of this tile
+#pragma unroll 2
+      for (int k = 0; k < AF_KEYS; k += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(pr + i * 4 * AF_SPITCH + k);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          ulonglong2 v[NJ];
+#pragma unroll
+          for (int j = 0; j < NJ; ++j)
+            if (NJ * 32 == d || tx * 4 + 32 * j < d) v[j] = af_lds2(vs + (k + u) * pitch + 32 * j);
+          if (every) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float pu = u == 0 ? p[i].x : u == 1 ? p[i].y : u == 2 ? p[i].z : p[i].w;
+              const f32x2 pp = af_pair(pu, pu);
+#pragma unroll
+              for (int j = 0; j < NJ; ++j) {
+                a[i][2 * j] = af_fma2(pp, v[j].x, a[i][2 * j]);
+                a[i][2 * j + 1] = af_fma2(pp, v[j].y, a[i][2 * j + 1]);
+              }
+            }
+          } else {
+            // a hidden key adds nothing, whatever stands in its value (0 times an infinity would)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int key = k0 + k + u;
+              const bool seen = key <= pos[i] && (A.window <= 0 || key > pos[i] - A.window);
+              const float pu = u == 0 ? p[i].x : u == 1 ? p[i].y : u == 2 ? p[i].z : p[i].w;
+              const f32x2 pp = af_pair(pu, pu);
+#pragma unroll
+              for (int j = 0; j < NJ; ++j) {
+                const f32x2 x = af_fma2(pp, v[j].x, a[i][2 * j]), y = af_fma2(pp, v[j].y, a[i][2 * j + 1]);
+                a[i][2 * j] = seen ? x : a[i][2 * j];
+                a[i][2 * j + 1] = seen ? y : a[i][2 * j + 1];
+              }
+            }
+          }
+        }
+      }
+      buf ^= 1;
+    }
+    // ---- the range joins the total ----
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (rm[i] == -INFINITY) continue;                                        // the row sees no key of this range
+      float c1, c2;
+      af_weights(m[i], l[i], rm[i], rl[i], c1, c2);
+#pragma unroll
+      for (int j = 0; j < NJ * 2; ++j) {
+        const float2 t = af_split(total[i][j]), v = af_split(a[i][j]);
+        total[i][j] = af_pair(fmaf(t.x, c1, v.x * c2), fmaf(t.y, c1, v.y * c2));
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + warp * 16 + ty + 4 * i;
+    if (row >= n_rows) continue;
+    const int token = row / g, head = kvh * g + row - token * g;
+    float* o = A.out + (size_t)(tok0 + token) * A.nq * d + (size_t)head * d + tx * 4;
+    const float inv = 1.0f / l[i];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      if (NJ * 32 != d && tx * 4 + 32 * j >= d) continue;
+      const float2 x = af_split(total[i][2 * j]), y = af_split(total[i][2 * j + 1]);
+      *reinterpret_cast<float4*>(o + 32 * j) = make_float4(x.x * inv, x.y * inv, y.x * inv, y.y * inv);
+    }
+  }
+}
+
+// ---- entries of one token ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(AF_THREADS) af32_single_kernel(const Af32Args A) {
+  extern __shared__ __align__(16) float af_smem[];
+  const int d = A.d, pitch = d + 4, g = A.nq / A.nkv;
+  float* ks = af_smem;                                          // [128 keys][pitch]
+  float* vs = ks + AF_RANGE * pitch;                            // [128 keys][d]
+  float* qs = vs + AF_RANGE * d;                                // [AF_HEADS][d]
+  float* ps = qs + AF_HEADS * d;                                // [AF_HEADS][128]
+  float* stats = ps + 2 * AF_HEADS * AF_RANGE;                  // maximum and sum of every row (the room between: factors, below)
+  __shared__ unsigned long long places[AF_RANGE];
+  __shared__ int is_last;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int entry = blockIdx.z, kvh = blockIdx.y;
+  pdl_trigger();
+  const int token = A.cu_q[entry];
+  const bool single = A.cu_q[entry + 1] - token == 1;
+  const int p = A.start[entry], lo = A.window > 0 ? max(0, p - A.window + 1) : 0;
+  const int r_first = lo / AF_RANGE, r_last = p / AF_RANGE, range = r_first + (int)blockIdx.x;
+  pdl_wait();
+  if (!single || range > r_last) return;
+  const int base = range * AF_RANGE, k_lo = max(0, lo - base), k_hi = min(AF_RANGE - 1, p - base);
+  const int* table = A.table + (size_t)entry * A.table_width;
+  const int chunks = d >> 2;
+  {
+    const int at = base + min(max(tid, k_lo), k_hi);
+    places[tid] = (((unsigned long long)table[at / A.page_size] * A.nkv + kvh) * A.page_size + at % A.page_size) * d;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int i = tid; i < (k_hi + 1) * chunks; i += AF_THREADS) {
+    const int k = i / chunks, c = i - k * chunks;
+    const unsigned long long off = places[k] + c * 4;
+    af_copy16(ks + k * pitch + c * 4, A.kpages + off, k >= k_lo);
+    af_copy16(vs + k * d + c * 4, A.vpages + off, k >= k_lo);
+  }
+  af_commit();
+  const float* q = A.qkv + (size_t)token * A.qkv_stride + (size_t)kvh * g * d;
+  float* o = A.out + (size_t)token * A.nq * d + (size_t)kvh * g * d;
+  const int ranges = r_last - r_first + 1;
+  float* part = A.scratch + ((((size_t)entry * A.nkv + kvh) * A.ranges) * g) * (d + 2);     // [range][head][d + 2]
+  float* mine = part + (size_t)blockIdx.x * g * (d + 2);
+  for (int h0 = 0; h0 < g; h0 += AF_HEADS) {
+    const int nh = min(AF_HEADS, g - h0);
+    for (int i = tid; i < AF_HEADS * d; i += AF_THREADS) qs[i] = i < nh * d ? q[h0 * d + i] : 0.f;
+    af_wait<0>();
+    __syncthreads();
+    {                                                           // a key a thread
+      f32x2 s[AF_HEADS];
+#pragma unroll
+      for (int h = 0; h < AF_HEADS; ++h) s[h] = 0;
+      if (tid >= k_lo && tid <= k_hi)
+#pragma unroll 4
+        for (int c = 0; c < chunks; ++c) {
+          const ulonglong2 k = af_lds2(ks + tid * pitch + c * 4);
+#pragma unroll
+          for (int h = 0; h < AF_HEADS; ++h) {
+            const ulonglong2 x = af_lds2(qs + h * d + c * 4);
+            s[h] = af_fma2(x.x, k.x, s[h]);
+            s[h] = af_fma2(x.y, k.y, s[h]);
+          }
+        }
+#pragma unroll
+      for (int h = 0; h < AF_HEADS; ++h) {
+        const float2 v = af_split(s[h]);
+        ps[h * AF_RANGE + tid] = tid >= k_lo && tid <= k_hi ? (v.x + v.y) * A.scale : -INFINITY;
+      }
+    }
+    __syncthreads();
+    for (int h = warp; h < nh; h += AF_THREADS / 32) {
+      float* row = ps + h * AF_RANGE;
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = row[lane + 32 * j];
+      const float top = warp_max(fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])));
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = v[j] == -INFINITY ? 0.f : expf(v[j] - top);
+        row[lane + 32 * j] = e;
+        sum += e;
+      }
+      sum = warp_sum(sum);
+      if (lane == 0) { stats[2 * h] = top; stats[2 * h + 1] = sum; }
+    }
+    __syncthreads();
+    if (tid < d) {                                              // a channel a thread
+      float a[AF_HEADS];
+#pragma unroll
+      for (int h = 0; h < AF_HEADS; ++h) a[h] = 0.f;
+      const float* v = vs + tid;
+      int k = k_lo;
+      for (; k + 3 <= k_hi && k % 4 == 0; k += 4) {
+        const float v0 = v[k * d], v1 = v[(k + 1) * d], v2 = v[(k + 2) * d], v3 = v[(k + 3) * d];
+#pragma unroll
+        for (int h = 0; h < AF_HEADS; ++h) {
+          const float4 e = *reinterpret_cast<const float4*>(ps + h * AF_RANGE + k);
+          a[h] = fmaf(e.w, v3, fmaf(e.z, v2, fmaf(e.y, v1, fmaf(e.x, v0, a[h]))));
+        }
+      }
+      for (; k <= k_hi; ++k) {
+        const float v0 = v[k * d];
+#pragma unroll
+        for (int h = 0; h < AF_HEADS; ++h) a[h] = fmaf(ps[h * AF_RANGE + k], v0, a[h]);
+      }
+#pragma unroll
+      for (int h = 0; h < AF_HEADS; ++h) {
+        if (h >= nh) continue;
+        if (ranges == 1) o[(h0 + h) * d + tid] = a[h] * (1.0f / stats[2 * h + 1]);
+        else mine[(size_t)(h0 + h) * (d + 2) + tid] = a[h];
+      }
+    }
+    if (ranges > 1 && tid < 2 * nh) mine[(size_t)(h0 + (tid >> 1)) * (d + 2) + d + (tid & 1)] = stats[tid];
+    __syncthreads();
+  }
+  if (ranges == 1) return;
+  // ---- the CTA that comes last adds the ranges up, in order ----
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    int* counter = A.counters + entry * A.nkv + kvh;
+    is_last = atomicAdd(counter, 1) == ranges - 1;
+    if (is_last) *counter = 0;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  // The factors of AF_RANGE ranges at a time for AF_HEADS heads, a thread a head, then the values: their loads depend on nothing.
+  float2* factors = reinterpret_cast<float2*>(ps);                              // [AF_HEADS][AF_RANGE]
+  for (int h0 = 0; h0 < g; h0 += AF_HEADS) {
+    const int nh = min(AF_HEADS, g - h0);
+    float m = -INFINITY, l = 0.f;                                               // of head h0 + tid
+    float total[AF_HEADS];
+#pragma unroll
+    for (int h = 0; h < AF_HEADS; ++h) total[h] = 0.f;
+    for (int r0 = 0; r0 < ranges; r0 += AF_RANGE) {
+      const int nr = min(AF_RANGE, ranges - r0);
+      __syncthreads();
+      for (int i = tid; i < nh * nr; i += AF_THREADS) {
+        const int h = i / nr, r = i - h * nr;
+        factors[h * AF_RANGE + r] = __ldcg(reinterpret_cast<const float2*>(part + ((size_t)(r0 + r) * g + h0 + h) * (d + 2) + d));
+      }
+      __syncthreads();
+      if (tid < nh)
+        for (int r = 0; r < nr; ++r) {
+          const float2 v = factors[tid * AF_RANGE + r];
+          float c1 = 1.f, c2 = -1.f;                                            // a range without a visible key is left out
+          if (v.x != -INFINITY) af_weights(m, l, v.x, v.y, c1, c2);
+          factors[tid * AF_RANGE + r] = make_float2(c1, c2);
+        }
+      __syncthreads();
+      if (tid < d)
+#pragma unroll
+        for (int h = 0; h < AF_HEADS; ++h) {
+          if (h >= nh) continue;
+          const float* src = part + ((size_t)r0 * g + h0 + h) * (d + 2) + tid;
+#pragma unroll 8
+          for (int r = 0; r < nr; ++r) {
+            const float a = __ldcg(src + (size_t)r * g * (d + 2));
+            const float2 c = factors[h * AF_RANGE + r];
+            total[h] = c.y < 0.f ? total[h] : fmaf(total[h], c.x, a * c.y);
+          }
+        }
+    }
+    if (tid < nh) stats[tid] = l;
+    __syncthreads();
+    if (tid < d)
+#pragma unroll
+      for (int h = 0; h < AF_HEADS; ++h)
+        if (h < nh) o[(size_t)(h0 + h) * d + tid] = total[h] * (1.0f / stats[h]);
+  }
+}
+
+// singles: entries of one token go to their own kernel (else they are runs); runs: there are others.  scratch: entries * nq * ranges * (d + 2) floats when
+// ranges (the most ranges of 128 keys an entry's visible keys can touch) > 1; counters: entries * nkv zeroed ints.
+Q25_EXPORT int q25_paged_attention_f32(const float* qkv, int qkv_stride, float* out, const float* kpages, const float* vpages,
+                                       const int* block_table, int table_width, const int* cu_q, const int* q_start_pos, int n_tokens,
+                                       int entries, int nq, int nkv, int d, int page_size, int window, float scale, int runs, int singles,
+                                       int ranges, float* scratch, int* counters, void* stream) {
+  if (n_tokens <= 0 || entries <= 0) return 0;
+  if (d <= 0 || d > 128 || d % 16 || nkv <= 0 || nq % nkv || page_size <= 0 || qkv_stride % 4 || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) ||
+      ((uintptr_t)kpages & 15) || ((uintptr_t)vpages & 15) || ranges < 1 || nkv > 65535)
+    return (int)cudaErrorInvalidValue;
+  const Af32Args A = {qkv, out, kpages, vpages, block_table, cu_q, q_start_pos, qkv_stride, table_width, entries, nq, nkv, d, page_size, window,
+                      scale, singles ? 2 : 1, ranges, scratch, counters};
+  cudaStream_t s = (cudaStream_t)stream;
+  if (runs) {
+    const int g = nq / nkv;
+    const long long tiles = ((long long)n_tokens * g + AF_ROWS - 1) / AF_ROWS + (entries < n_tokens ? entries : n_tokens);      // at most
+    const int smem = (AF_ROWS * (d + 4) + AF_ROWS * AF_SPITCH + 2 * AF_KEYS * (d + 4)) * 4;
+#define AF_TILE(NJ)                                                                                                                     \
+  case NJ: {                                                                                                                            \
+    const cudaError_t e = cudaFuncSetAttribute(af32_tile_kernel<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);          \
+    if (e != cudaSuccess) return (int)e;                                                                                                \
+    launch(af32_tile_kernel<NJ>, dim3((unsigned)tiles, nkv), dim3(AF_THREADS), smem, s, A);                                             \
+    break;                                                                                                                              \
+  }
+    switch ((d + 31) / 32) { AF_TILE(1) AF_TILE(2) AF_TILE(3) AF_TILE(4) }
+#undef AF_TILE
+  }
+  if (singles) {
+    if (entries > 65535 || (ranges > 1 && (!scratch || !counters))) return (int)cudaErrorInvalidValue;
+    const int smem = (AF_RANGE * (d + 4) + AF_RANGE * d + AF_HEADS * d + 2 * AF_HEADS * AF_RANGE + 2 * AF_HEADS) * 4;
+    const cudaError_t e = cudaFuncSetAttribute(af32_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 150 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    launch(af32_single_kernel, dim3(ranges, nkv, entries), dim3(AF_THREADS), smem, s, A);
+  }
+  return launch_status();
+}

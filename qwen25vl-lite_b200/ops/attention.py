@@ -9,8 +9,8 @@ bfloat16 with a head size and page size the tensor-core kernels take (``csrc/att
   token go to the split-KV decode kernel (partials through scratch memory and a combine
   kernel) and runs of tokens to the prefill kernel (tcgen05 at head size 128, mma.sync else).
 
-Everything else (float32, other sizes) goes to the general kernel
-(``csrc/attention_generic.cu``) after ``rotate_and_store``.
+float32 with heads of up to 128 channels goes to its own kernels (``csrc/attention_f32.cu``: tiles for runs, ranges of keys for
+single tokens), everything else to the general kernel (``csrc/attention_generic.cu``), both after ``rotate_and_store``.
 
 The tensor-core kernels walk work lists: the entries that bring one token, and (entry, row tile)
 pairs for the others.  ``plan_step`` builds them on the host from the step's shape; the step
@@ -194,6 +194,17 @@ def _scratch_floats(n: int, device, use: str = "decode") -> torch.Tensor:
     return buf
 
 
+# The single tokens' partial results of the 32-bit attention may take this much (256 MB); where they would take more (256 requests
+# at 60,000 keys each, 16 heads of 128) the tile kernel takes the single tokens too, slower for them and without scratch memory.
+F32_SCRATCH_MOST = 1 << 26
+
+
+def f32_ranges(max_kv_len: int, window: int) -> int:
+    """The most ranges of keys that one query's visible keys can touch."""
+    ranges = -(-max_kv_len // kernels.F32_RANGE)
+    return max(1, min(ranges, (window - 2) // kernels.F32_RANGE + 2) if window else ranges)
+
+
 def _pairs(flat, width: int = 2):
     return None if flat is None else flat.view(-1, width)
 
@@ -248,6 +259,19 @@ def paged_attention(ctx, plan, qkv, kv, nq: int, nkv: int, head_dim: int, window
         out = torch.empty((qkv.shape[0], nq * head_dim), dtype=qkv.dtype, device=qkv.device)
     window = int(window or 0)
     group = nq // nkv
+    if kernels.paged_attention_f32_supports(qkv, head_dim):
+        singles, ranges, scratch = 1 in ctx.host_q_lens, 1, None
+        if singles:
+            ranges = f32_ranges(ctx.max_kv_len, window)
+            floats = ctx.n_seqs * nq * ranges * (head_dim + 2)
+            if ranges > 1 and floats > F32_SCRATCH_MOST:
+                singles = False
+            elif ranges > 1:
+                scratch = _scratch_floats(floats, qkv.device)
+        kernels.paged_attention_f32(qkv, out, kv.k_pages, kv.v_pages, kv.block_table, ctx.cu_q, ctx.q_start_pos, ctx.n_seqs, nq, nkv,
+                                    head_dim, kv.page_size, window, scale, runs=not singles or ctx.max_q_len > 1, singles=singles,
+                                    ranges=ranges, scratch=scratch)
+        return out
     if not kernels.attention_mma_supports(qkv.dtype, head_dim, kv.page_size):
         kernels.paged_attention_generic(qkv, out, kv.k_pages, kv.v_pages, kv.block_table, ctx.token_seq, ctx.cu_q,
                                         ctx.q_start_pos, nq, nkv, head_dim, kv.page_size, window, scale)

@@ -66,6 +66,7 @@ _UNTYPED = {
     "q25_attention_prefill_bf16": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P],
     "q25_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P, _P],
     "q25_gemm_tcgen05_bf16": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P],
+    "q25_paged_attention_f32": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P],
     "q25_sample_rows": [_P, _LL, _I, _I, _P, _P, _P, _P, _P, _P],
     "q25_apply_penalties": [_P, _LL, _I, _I, _P, _P, _P, _P, _P, _P, _P],
 }
@@ -265,6 +266,37 @@ def paged_attention_generic(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch
         page_size, int(window or 0), float(scale), _stream()), "paged_attention_generic")
 
 
+F32_RANGE = 128                 # keys of one range of the 32-bit attention
+
+
+def paged_attention_f32_supports(qkv: torch.Tensor, head_dim: int) -> bool:
+    """What the tiled 32-bit attention takes; other sizes and layouts go to the general kernel."""
+    return (qkv.dtype == torch.float32 and head_dim % 16 == 0 and 16 <= head_dim <= 128 and qkv.stride(1) == 1
+            and qkv.stride(0) % 4 == 0 and qkv.data_ptr() % 16 == 0)
+
+
+def paged_attention_f32(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
+                        block_table: torch.Tensor, cu_q: torch.Tensor, q_start_pos: torch.Tensor, entries: int, nq: int, nkv: int,
+                        head_dim: int, page_size: int, window: int, scale: float, runs: bool, singles: bool, ranges: int = 1,
+                        scratch: Optional[torch.Tensor] = None) -> None:
+    """``paged_attention_generic`` in float32 on tiles.  ``singles``: the entries of one token go to a kernel of their own, which
+    cuts their visible keys into ranges of ``F32_RANGE`` (at most ``ranges`` each; with more than one, partial results go through
+    ``scratch``, float32, entries * nq * ranges * (head_dim + 2)); ``runs``: there are entries for the other kernel (without
+    ``singles`` it takes all).  A query gets the same bits from either."""
+    if not paged_attention_f32_supports(qkv, head_dim) or not out.is_contiguous():
+        raise KernelError(f"paged_attention_f32: unsupported head size {head_dim} or layout")
+    if singles and ranges > 1 and (scratch is None or scratch.dtype != torch.float32
+                                   or scratch.numel() < entries * nq * ranges * (head_dim + 2)):
+        raise KernelError(f"paged_attention_f32: {ranges} ranges need scratch memory")
+    _check(_fn("q25_paged_attention_f32", _UNTYPED["q25_paged_attention_f32"])(
+        qkv.data_ptr(), qkv.stride(0), out.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
+        block_table.shape[1], cu_q.data_ptr(), q_start_pos.data_ptr(), qkv.shape[0], entries, nq, nkv, head_dim, page_size,
+        int(window or 0), float(scale), int(runs), int(singles), int(ranges), _ptr(scratch),
+        _split_counters(qkv.device, entries * nkv).data_ptr(), _stream()), "paged_attention_f32")
+    if runs and singles:
+        count_replayed(1)                      # two kernels by one call
+
+
 def attention_mma_supports(dtype: torch.dtype, head_dim: int, page_size: int) -> bool:
     """Sizes the tensor-core attention kernels take; everything else goes to the general kernel."""
     return (dtype == torch.bfloat16 and head_dim % 16 == 0 and 16 <= head_dim <= 128
@@ -346,12 +378,15 @@ def rope_angles(positions: torch.Tensor, inv_freq: torch.Tensor, axis: torch.Ten
 
 
 _counters: Dict[torch.device, torch.Tensor] = {}
+_counters_kept = []                            # smaller ones that captured steps may still point at
 
 
 def _split_counters(device, n: int) -> torch.Tensor:
     """Zeroed ints the fused decode attention counts its finished splits in (it leaves them zero)."""
     buf = _counters.get(device)
     if buf is None or buf.numel() < n:
+        if buf is not None:
+            _counters_kept.append(buf)
         buf = _counters[device] = torch.zeros(max(n, 4096), dtype=torch.int32, device=device)
     return buf
 

@@ -1,0 +1,59 @@
+"""The 32-bit attention on tiles and on ranges of keys: against the float64 oracle at the edges of tiles, ranges and windows,
+and bit for bit the same however the tokens are cut into entries and whichever kernel takes them."""
+
+import numpy as np
+import pytest
+import torch
+
+from test_kernels_gpu import attention_oracle, f64, paged_case, tol
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(c, lens, q_lens, nq, nkv, d, page_size, window, singles):
+    from qwen25vl_lite.ops import attention, kernels
+    singles = singles and 1 in q_lens
+    ranges = attention.f32_ranges(max(lens), window or 0)
+    scratch = torch.empty(len(lens) * nq * ranges * (d + 2), device="cuda")
+    out = torch.full((c["qkv"].shape[0], nq * d), float("nan"), device="cuda")
+    kernels.paged_attention_f32(c["qkv"], out, c["k_pages"], c["v_pages"], c["table"], c["cu"], c["start"], len(lens), nq, nkv, d,
+                                page_size, window or 0, d ** -0.5, max(q_lens) > 1 or not singles, singles, ranges, scratch)
+    return out
+
+
+@pytest.mark.parametrize("nq,nkv,d,page_size,window", [
+    (16, 2, 128, 16, None), (7, 1, 128, 16, 130), (4, 2, 16, 4, None), (6, 1, 32, 8, 1), (5, 5, 48, 16, 24), (3, 3, 80, 7, 40),
+    (20, 1, 64, 32, 128), (12, 6, 112, 16, 129)])
+def test_paged_attention_f32(nq, nkv, d, page_size, window):
+    rng = np.random.default_rng(nq * d)
+    # first tokens, whole prompts and portions that end beside a tile's and a range's edge, single tokens with one range and more
+    lens = [1, 37, 130, 128, 129, 257, 300, 64, 33, 2, 520]
+    q_lens = [1, 37, 2, 1, 1, 1, 45, 1, 33, 2, 260]
+    c = paged_case(rng, lens, q_lens, nq, nkv, d, page_size, torch.float32)
+    out = _run(c, lens, q_lens, nq, nkv, d, page_size, window, True)
+    assert np.abs(f64(out) - attention_oracle(c["dense"], window)).max() < tol(torch.float32)
+    assert torch.equal(_run(c, lens, q_lens, nq, nkv, d, page_size, window, False), out)
+    # every token an entry of its own: the same keys through the same pages
+    cu, starts = c["cu"].tolist(), c["start"].tolist()
+    own = dict(c, table=c["table"][c["token_seq"].long()].contiguous(), cu=torch.arange(cu[-1] + 1, dtype=torch.int32, device="cuda"),
+               start=torch.tensor([s + j for s, n in zip(starts, q_lens) for j in range(n)], dtype=torch.int32, device="cuda"))
+    n = cu[-1]
+    assert torch.equal(_run(own, [max(lens)] * n, [1] * n, nq, nkv, d, page_size, window, True), out)
+
+
+def test_paged_attention_f32_hidden_infinity():
+    """An infinity in the value of a later token, or of one that a window hides, reaches nobody who does not see it."""
+    rng = np.random.default_rng(3)
+    nq, nkv, d, ps, window = 4, 2, 64, 16, 50
+    lens, q_lens = [200], [150]
+    c = paged_case(rng, lens, q_lens, nq, nkv, d, ps, torch.float32)
+    for singles in (True, False):
+        clean = _run(c, lens, q_lens, nq, nkv, d, ps, window, singles)
+        key = 120
+        page = int(c["table"][0, key // ps])
+        v = c["v_pages"].clone()
+        v[page, :, key % ps] = float("inf")
+        out = _run(dict(c, v_pages=v), lens, q_lens, nq, nkv, d, ps, window, singles)
+        seen = torch.arange(50, 200) >= key
+        seen &= torch.arange(50, 200) < key + window
+        assert torch.equal(out[~seen], clean[~seen]) and not bool(torch.isfinite(out[seen]).any())
