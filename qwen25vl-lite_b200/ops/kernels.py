@@ -68,6 +68,7 @@ _UNTYPED = {
     "q25_gemm_tcgen05_bf16": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "q25_paged_attention_f32": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P],
     "q25_sample_rows": [_P, _LL, _I, _I, _P, _P, _P, _P, _P, _P],
+    "q25_sample_filtered": [_P, _LL, _I, _I, _P, _P, _P, _P],
     "q25_apply_penalties": [_P, _LL, _I, _I, _P, _P, _P, _P, _P, _P, _P],
 }
 
@@ -703,6 +704,27 @@ def sample_rows(logits: torch.Tensor, temperature: Optional[torch.Tensor], seed:
     _check(_fn("q25_sample_rows", _UNTYPED["q25_sample_rows"])(
         logits.data_ptr(), logits.stride(0), rows, vocab, _ptr(temperature), _ptr(seed), _ptr(token_index),
         out.data_ptr(), _ptr(scratch), _stream()), "sample_rows")
+
+
+SAMPLE_ASK_WORDS = 12           # 32-bit words of one row's ``SampleRow`` (csrc/sampling.cu)
+
+
+def sample_filtered_supports(logits: torch.Tensor) -> bool:
+    """Rows the one-launch sampler holds in the shared memory of a cluster."""
+    return (logits.is_cuda and logits.dtype == torch.float32 and logits.stride(1) == 1 and logits.shape[0] <= 65535
+            and 0 < logits.shape[1] <= _fn("q25_sample_filtered_most", [])())
+
+
+def sample_filtered(logits: torch.Tensor, asks: torch.Tensor, out: torch.Tensor) -> None:
+    """Penalties, top-k, min-p, top-p and the draw for every row.  ``asks`` (int32): ``SAMPLE_ASK_WORDS`` words a row, behind
+    them the rows' earlier tokens that those words point into.  ``logits`` are left as they are."""
+    rows, vocab = logits.shape
+    _dev(asks, torch.int32, "sample_filtered asks"); _dev(out, torch.int32, "sample_filtered out")
+    if not sample_filtered_supports(logits) or asks.numel() < rows * SAMPLE_ASK_WORDS or out.numel() < rows:
+        raise KernelError(f"sample_filtered: unsupported logits {tuple(logits.shape)} or too few words")
+    at = asks.data_ptr()
+    _check(_fn("q25_sample_filtered", _UNTYPED["q25_sample_filtered"])(
+        logits.data_ptr(), logits.stride(0), rows, vocab, at, at + 4 * rows * SAMPLE_ASK_WORDS, out.data_ptr(), _stream()), "sample_filtered")
 
 
 def apply_penalties(logits: torch.Tensor, ids: torch.Tensor, counts: torch.Tensor, offsets: torch.Tensor,

@@ -4,10 +4,11 @@ Order of operations as in the reference (src/qwen25vl_lite/sampling.py:44-106;
 src/qwen25vl_lite/engine.py:813-821): penalties on the logits, then for temperature > 0
 ``scores = logits / T``, top-k, min-p, top-p, softmax and one draw; temperature 0 is argmax.
 
-Greedy rows, plain temperature rows and penalties run in the engine's own kernels
-(``csrc/sampling.cu``), all rows of a step in one launch.  A row that asks for top-k, min-p
-or top-p is first narrowed with device-side sort and scan primitives and then drawn by the
-same kernel.  The draw is keyed by ``(seed, index of the token being drawn)`` like the
+Everything runs in the engine's own kernels (``csrc/sampling.cu``), all rows of a step in one
+launch: greedy and plain temperature rows in one that scans the logits, and steps in which a row
+asks for penalties, top-k, min-p or top-p in one that holds a row in a cluster's shared memory.
+Only rows of a vocabulary too large for that (above 400,000 tokens) are narrowed row by row with
+device-side sort and scan primitives.  The draw is keyed by ``(seed, index of the token being drawn)`` like the
 reference's ``seed + len(outputs)`` generator (engine.py:823-829); a request without a seed
 gets a fresh random one.
 """
@@ -15,6 +16,7 @@ gets a fresh random one.
 from __future__ import annotations
 
 import secrets
+from array import array
 from collections import Counter
 from typing import List, Optional, Sequence
 
@@ -92,6 +94,10 @@ class Sampler:
         rows = logits.shape[0]
         if rows == 0:
             return None
+        if any(p.has_penalties or p.has_filters for p in params) and kernels.sample_filtered_supports(logits):
+            out = torch.empty(rows, dtype=torch.int32, device=self.device)
+            kernels.sample_filtered(logits, self._asks(params, seeds, token_indices, previous), out)
+            return self._copy_back(out, rows)
         if any(p.has_penalties for p in params):
             logits = logits.clone()
             ids: List[int] = []
@@ -125,6 +131,42 @@ class Sampler:
             kernels.sample_rows(logits, self._upload(temps, torch.float32),
                                 torch.from_numpy(seed_arr).to(self.device, non_blocking=True),
                                 self._upload([int(t) for t in token_indices], torch.int32), out)
+        return self._copy_back(out, rows)
+
+    def _asks(self, params, seeds, token_indices, previous) -> torch.Tensor:
+        """What every row asks for, as the kernel reads it (``SampleRow``), and behind it the earlier tokens of the rows
+        with penalties as they came: the kernel counts them.  One copy from pinned memory."""
+        rows = len(params)
+        lists = array("i")
+        spans = []
+        for p, prev in zip(params, previous or [()] * rows):
+            begin = len(lists)
+            if p.has_penalties and prev:
+                lists.extend(prev)
+            spans.append((begin, len(lists)))
+        spans += [(len(lists), len(lists))] * (rows - len(spans))
+        words = rows * kernels.SAMPLE_ASK_WORDS
+        staged = torch.empty(words + max(len(lists), 1), dtype=torch.int32, pin_memory=True)
+        host = staged.numpy()
+        asks = host[:words].reshape(rows, kernels.SAMPLE_ASK_WORDS)
+        floats = asks.view(np.float32)
+        filters = [p.has_filters for p in params]
+        asks[:, 1] = [min(int(p.top_k or 0), 1 << 30) if f else 0 for p, f in zip(params, filters)]
+        floats[:, 0] = [p.temperature for p in params]
+        floats[:, 2] = [p.min_p if f else 0.0 for p, f in zip(params, filters)]
+        floats[:, 3] = [p.top_p if f else 1.0 for p, f in zip(params, filters)]
+        seed = np.array([int(s) & ((1 << 64) - 1) for s in seeds], dtype=np.uint64)
+        asks[:, 4] = seed.astype(np.uint32).view(np.int32)
+        asks[:, 5] = (seed >> np.uint64(32)).astype(np.uint32).view(np.int32)
+        asks[:, 6] = [int(t) for t in token_indices]
+        floats[:, 7] = [p.repetition_penalty for p in params]
+        floats[:, 8] = [p.presence_penalty for p in params]
+        floats[:, 9] = [p.frequency_penalty for p in params]
+        asks[:, 10:12] = spans
+        host[words:words + len(lists)] = np.frombuffer(lists, dtype=np.int32) if lists else 0
+        return staged.to(self.device, non_blocking=True)
+
+    def _copy_back(self, out: torch.Tensor, rows: int):
         if self.device.type != "cuda":
             return out.tolist(), None, rows, out
         if self._host is None or self._host.numel() < rows:

@@ -1,0 +1,63 @@
+"""The one-launch sampler against the plain implementation: every filter alone and together, rows of different wishes in one
+step, ties, vocabularies at the edges of the slices, penalties over long lists."""
+
+import numpy as np
+import pytest
+import torch
+
+from plain import decoder as plain
+
+pytestmark = pytest.mark.gpu
+
+WISHES = [dict(top_k=1), dict(top_k=20), dict(top_k=5000), dict(top_p=0.3), dict(top_p=0.95), dict(top_p=0.9999), dict(min_p=0.05),
+          dict(min_p=1.0), dict(top_k=50, min_p=0.02, top_p=0.8), dict(top_k=10 ** 9, top_p=0.5), dict()]
+
+
+def _rows(rng, rows, vocab, kind):
+    if kind == "flat":                             # every score alike but for a few: the searches end in ties
+        x = np.zeros((rows, vocab), dtype=np.float32)
+        x[:, :: max(1, vocab // 7)] = 0.5
+        return x
+    x = rng.standard_normal((rows, vocab)).astype(np.float32) * 2
+    if kind == "peaks":
+        x[np.arange(rows)[:, None], rng.integers(0, vocab, (rows, 40))] += 12
+    if kind == "coarse":                           # few different scores, many ties
+        x = np.round(x)
+    return x
+
+
+@pytest.mark.parametrize("vocab,kind", [(1, "normal"), (7, "normal"), (31, "coarse"), (300, "normal"), (4099, "flat"), (32000, "peaks"),
+                                        (32000, "normal"), (32001, "coarse"), (151936, "peaks"), (152064, "normal")])
+def test_sample_filtered(vocab, kind):
+    from qwen25vl_lite.sampling import Sampler, SamplingParams
+    rng = np.random.default_rng(vocab)
+    logits = _rows(rng, len(WISHES) + 2, vocab, kind)
+    params = [SamplingParams(temperature=0.7, **w) for w in WISHES] + [SamplingParams(), SamplingParams(temperature=1.3)]
+    seeds = [int(s) for s in rng.integers(0, 1 << 63, len(params))]
+    index = list(range(3, 3 + len(params)))
+    got = Sampler("cuda").sample(torch.tensor(logits, device="cuda"), params, seeds, index, [[]] * len(params))
+    for r, p in enumerate(params):
+        # a filtered row's scores are multiplied by 1 / T; the plain implementation divides
+        scaled = logits[r] * (np.float32(1.0) / np.float32(p.temperature)) if p.has_filters else logits[r]
+        t = 1.0 if p.has_filters else p.temperature
+        want = plain.sample(scaled, t, seeds[r], index[r], max(p.top_k, -1), p.min_p, p.top_p)
+        assert got[r] == want, (r, p)
+
+
+def test_sample_filtered_penalties():
+    from qwen25vl_lite.sampling import Sampler, SamplingParams
+    rng = np.random.default_rng(1)
+    vocab = 5003
+    prev = [[], [17], rng.integers(0, 40, 300).tolist(), rng.integers(0, vocab, 9000).tolist(), [5] * 70000, [3, 3, 9]]
+    params = [SamplingParams(repetition_penalty=1.2), SamplingParams(repetition_penalty=2.0, presence_penalty=0.5),
+              SamplingParams(frequency_penalty=0.05, repetition_penalty=0.9), SamplingParams(temperature=0.8, presence_penalty=1.5, top_p=0.7),
+              SamplingParams(temperature=0.5, frequency_penalty=1e-4, top_k=30), SamplingParams(temperature=0.9, top_k=5)]
+    logits = _rows(rng, len(params), vocab, "peaks")
+    before = torch.tensor(logits, device="cuda")
+    given = before.clone()
+    got = Sampler("cuda").sample(given, params, list(range(6)), [4] * 6, prev)
+    assert torch.equal(given, before)
+    for r, p in enumerate(params):
+        row = plain.apply_penalties(logits[r], prev[r], p.repetition_penalty, p.presence_penalty, p.frequency_penalty)
+        want = plain.sample(row, p.temperature, r, 4, p.top_k, p.min_p, p.top_p)
+        assert got[r] == want, (r, p)
