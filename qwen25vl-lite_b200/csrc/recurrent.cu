@@ -103,13 +103,14 @@ rglru_gates_kernel(const float* __restrict__ u, const float* __restrict__ ra, co
 // The same for steps of few tokens (decode): a CTA takes 16 tokens x 16 channels of one block and
 // brings the whole depth of the product into shared memory at once, so that all its loads are in
 // flight together instead of a chain of tiles; one thread per (token, channel), the same FMA chains
-// in the same order as above.  Dynamic shared memory: 3 x bw x 17 floats.
+// in the same order as above.  Dynamic shared memory: 3 x bw x 17 floats.  The matrices and vectors, which no
+// kernel writes, are fetched before the wait for the kernel before (8 tokens of 2,048 channels in 16 blocks add 9.6 us to a
+// step instead of 12.5).
 __global__ void __launch_bounds__(256)
 rglru_gates_small_kernel(const float* __restrict__ u, const float* __restrict__ ra, const float* __restrict__ ra_b,
                          const float* __restrict__ ri, const float* __restrict__ ri_b, const float* __restrict__ lam,
                          float gain, float* __restrict__ a_out, float* __restrict__ bx_out, int n_tokens, int width, int bw) {
   pdl_trigger();
-  pdl_wait();
   extern __shared__ float gates_smem[];
   float* Us = gates_smem;                  // [bw][17]
   float* As = Us + (size_t)bw * 17;
@@ -117,30 +118,37 @@ rglru_gates_small_kernel(const float* __restrict__ u, const float* __restrict__ 
   const int b = blockIdx.z, m0 = blockIdx.y * 16, n0 = blockIdx.x * 16;
   const float* Wa = ra + (size_t)b * bw * bw;
   const float* Wi = ri + (size_t)b * bw * bw;
+#pragma unroll 8
   for (int e = threadIdx.x; e < 16 * bw; e += 256) {
     const int r = e / bw, k = e % bw;                     // consecutive threads read consecutive k
-    const int gm = m0 + r, gn = n0 + r;
-    Us[k * 17 + r] = gm < n_tokens ? u[(size_t)gm * width + b * bw + k] : 0.f;
+    const int gn = n0 + r;
     As[k * 17 + r] = gn < bw ? Wa[(size_t)gn * bw + k] : 0.f;
     Is[k * 17 + r] = gn < bw ? Wi[(size_t)gn * bw + k] : 0.f;
   }
-  __syncthreads();
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int gm = m0 + ty, gn = n0 + tx, c = b * bw + min(gn, bw - 1);
+  const float bias_a = ra_b[c], bias_i = ri_b[c], rate = softplus_f(lam[c]);
+  pdl_wait();
+#pragma unroll 8
+  for (int e = threadIdx.x; e < 16 * bw; e += 256) {
+    const int r = e / bw, k = e % bw;
+    Us[k * 17 + r] = m0 + r < n_tokens ? u[(size_t)(m0 + r) * width + b * bw + k] : 0.f;
+  }
+  __syncthreads();
   float acc_a = 0.f, acc_i = 0.f;
+#pragma unroll 8
   for (int k = 0; k < bw; ++k) {
     const float uu = Us[k * 17 + ty];
     acc_a = fmaf(uu, As[k * 17 + tx], acc_a);
     acc_i = fmaf(uu, Is[k * 17 + tx], acc_i);
   }
-  const int gm = m0 + ty, gn = n0 + tx;
   if (gm >= n_tokens || gn >= bw) return;
-  const int c = b * bw + gn;
-  const float r = sigmoid_f(acc_a + ra_b[c]);
-  const float g = sigmoid_f(acc_i + ri_b[c]);
-  const float log_a = -gain * r * softplus_f(lam[c]);
+  const float r = sigmoid_f(acc_a + bias_a);
+  const float g = sigmoid_f(acc_i + bias_i);
+  const float log_a = -gain * r * rate;
   const size_t at = (size_t)gm * width + c;
   a_out[at] = expf(log_a);
-  bx_out[at] = sqrtf(-expm1f(2.0f * log_a)) * g * u[at];
+  bx_out[at] = sqrtf(-expm1f(2.0f * log_a)) * g * Us[gn * 17 + ty];
 }
 
 // Both gates for long steps on tensor cores (mma.sync, float accumulators), for gate matrices whose entries are bfloat16
