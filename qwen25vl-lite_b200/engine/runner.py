@@ -203,7 +203,7 @@ class ModelRunner:
         self._capture_stream = None
         self._graph_pool = None
         self.graph_replays = 0
-        # kernels with bounded waits report a wait that gave up here; read back after every step
+        # kernels with bounded waits report a wait that gave up here; written behind every step's kernels
         # and looked at before the next one
         self._error_host = torch.zeros(1, dtype=torch.int32, pin_memory=self.device.type == "cuda")
 
@@ -294,12 +294,15 @@ class ModelRunner:
         into single persistent kernels (``kernels.chain_begin``).  Only for steps whose forward
         launches nothing but this engine's kernels, which is what ``graph_safe`` parts promise."""
         if self.dtype != torch.bfloat16:                  # the 32-bit path has no weight-streaming products
-            return self.model.forward(ctx)
-        kernels.chain_begin()
-        try:
-            return self.model.forward(ctx)
-        finally:
-            kernels.chain_end()
+            logits = self.model.forward(ctx)
+        else:
+            kernels.chain_begin(zeroed=True)              # by the kernel that brought the step's arrays
+            try:
+                logits = self.model.forward(ctx)
+            finally:
+                kernels.chain_end()
+        kernels.step_end(self._device_ints.device, self._error_host)
+        return logits
 
     def step(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:
         """Runs the tokens the entries bring, as one batch.  Returns float32 logits
@@ -552,7 +555,10 @@ class ModelRunner:
                 raise ValueError(f"a prepared step needs {real} token ids in [0, {self.vocab_size})")
             tok[:real] = ids
         dev = self._device_ints
-        dev[:off].copy_(self._staging[:off], non_blocking=True)
+        if self.device.type == "cuda":
+            kernels.step_begin(self._staging, dev, off)
+        else:
+            dev[:off].copy_(self._staging[:off], non_blocking=True)
         if device_ids is not None:
             dev[tok_s[0]:tok_s[0] + real].copy_(device_ids[:real], non_blocking=True)
         if self._staging_free is not None:
@@ -579,6 +585,8 @@ class ModelRunner:
         try:
             if graph_key is None:
                 logits = self.model.forward(make_ctx())
+                if self.device.type == "cuda":
+                    kernels.step_end(self._device_ints.device, self._error_host)
             else:
                 logits = self._replay(graph_key, make_ctx, (dev.data_ptr(), off))
         finally:
@@ -588,8 +596,6 @@ class ModelRunner:
         if S > real:
             logits = logits[:real]
 
-        if self.device.type == "cuda":
-            self._error_host.copy_(kernels.error_flag(self.device), non_blocking=True)
         for e, n, p_max in zip(entries, q_lens, last_position):
             # where plain text that follows resumes is the position encoding's to say
             c = e.request.cache

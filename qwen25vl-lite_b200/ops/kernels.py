@@ -586,14 +586,16 @@ def chain_available() -> bool:
     return _chain_ok
 
 
-def chain_begin() -> bool:
+def chain_begin(zeroed: bool = False) -> bool:
     """Starts gathering.  The counter of the kernels' barrier starts from zero in every gathering
-    (a memset on the stream), so the values that a captured graph carries hold in every replay."""
+    (a memset on the stream, unless ``step_begin`` has just done it: ``zeroed``), so the values that a captured
+    graph carries hold in every replay."""
     global _chain, _chain_base
     if _chain is None and chain_available():
         _chain, _chain_base = [], 0
         device = torch.device("cuda", torch.cuda.current_device())
-        _chain_buffers(device)[1].zero_()
+        if not zeroed:
+            _chain_buffers(device)[1].zero_()
     return _chain is not None
 
 
@@ -676,6 +678,32 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
     _check(_fn("q25_gemm_tcgen05_bf16", _UNTYPED["q25_gemm_tcgen05_bf16"])(
         w.data_ptr(), x.data_ptr(), x.stride(0), _ptr(bias), out.data_ptr(), out.stride(0), m, n, k, int(epilogue),
         error_flag(x.device).data_ptr(), _stream()), "gemm_tcgen05")
+
+
+# A step's arrays up to this many ints travel by a kernel that reads pinned memory (64 KB: 16 us at the rate 148 SMs pull over
+# PCIe; a decode step of 64 requests at 2,000 keys has 10,000); more go by the copy engine, which is faster from there on.
+STEP_BEGIN_INTS = 16384
+
+
+def step_begin(staging: torch.Tensor, ints: torch.Tensor, n: int) -> None:
+    """A step's int arrays, the first ``n`` of ``staging`` (which the caller has allocated pinned), to the device, and the chain
+    kernels' barrier to zero."""
+    by_kernel, whole = n <= STEP_BEGIN_INTS, (n + 3) // 4 * 4
+    if staging.dtype != torch.int32 or ints.dtype != torch.int32 or staging.numel() < whole or ints.numel() < whole or not ints.is_cuda:
+        raise KernelError("step_begin: needs int32 buffers with room for the step's arrays in whole 16 bytes")
+    if not by_kernel:
+        ints[:n].copy_(staging[:n], non_blocking=True)
+    barrier = _chain_buffers(ints.device)[1]
+    _check(_fn("q25_step_begin", [_P, _P, _I, _P, _I, _P])(staging.data_ptr(), ints.data_ptr(), n if by_kernel else 0, barrier.data_ptr(),
+                                                           barrier.numel(), _stream()), "step_begin")
+
+
+def step_end(device, host: torch.Tensor) -> None:
+    """Behind a step's kernels: the code one of them may have left travels to the pinned ``host`` (int32 [1]); without one
+    nothing is written."""
+    if host.dtype != torch.int32:
+        raise KernelError("step_end: the host's flag is int32")
+    _check(_fn("q25_step_end", [_P, _P, _P])(error_flag(device).data_ptr(), host.data_ptr(), _stream()), "step_end")
 
 
 def reset_after_error(device) -> None:
