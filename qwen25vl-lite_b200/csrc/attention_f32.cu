@@ -12,7 +12,10 @@
 //     warp 16 of them; keys and values come in tiles of 32 through two buffers (cp.async), and both products are packed
 //     FMAs on registers (16 rows x 32 keys, then 16 rows x all channels for a warp);
 //   * af32_single_kernel: entries of one token.  A CTA takes one range of one kv head: a thread owns a key for the scores and a
-//     channel for the values; the CTA that finishes an entry's last range adds them all up.
+//     channel for the values, for two heads of eight; all keys but the token's own, which earlier steps wrote, are fetched
+//     before the wait for the kernel before; the CTA that finishes an entry's last range adds them all up.  (Bound by that
+//     chain of trips: it adds 10.5 us to a step at 100 keys, 15.7 with one set of 128 threads for all eight heads and no
+//     early fetch; 16 tokens at 1,500 keys 33 us instead of 49.5.)
 //
 // One warp per (token, head) on the CUDA cores with a key per lane, as before, read every key again for every row: 9.6 ms for
 // a prompt of 1,500 tokens with 16 heads of 128 (0.96 TFLOP/s), 750 us for one token at 1,500 keys.
@@ -23,7 +26,9 @@
 #define AF_ROWS 64                               // rows of a CTA of the tile kernel
 #define AF_THREADS 128
 #define AF_SPITCH 136                            // floats between rows of scores: four rows' stores lie in different banks
-#define AF_HEADS 8                               // rows the single kernel works on at a time
+#define AF_HEADS 8                               // heads the single kernel works on at a time, by
+#define AS_THREADS 512                           // four sets of 128 threads, each
+#define AS_PER (AF_HEADS * 128 / AS_THREADS)     // with its own
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 af_fma2(f32x2 a, f32x2 b, f32x2 c) {
@@ -312,7 +317,7 @@ __global__ void __launch_bounds__(AF_THREADS, 2) af32_tile_kernel(const Af32Args
 }
 
 // ---- entries of one token ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(AF_THREADS) af32_single_kernel(const Af32Args A) {
+__global__ void __launch_bounds__(AS_THREADS) af32_single_kernel(const Af32Args A) {
   extern __shared__ __align__(16) float af_smem[];
   const int d = A.d, pitch = d + 4, g = A.nq / A.nkv;
   float* ks = af_smem;                                          // [128 keys][pitch]
@@ -323,29 +328,39 @@ __global__ void __launch_bounds__(AF_THREADS) af32_single_kernel(const Af32Args 
   __shared__ unsigned long long places[AF_RANGE];
   __shared__ int is_last;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int at = tid & 127, hq = (tid >> 7) * AS_PER;           // this thread's key, then channel, and its heads
   const int entry = blockIdx.z, kvh = blockIdx.y;
   pdl_trigger();
   const int token = A.cu_q[entry];
   const bool single = A.cu_q[entry + 1] - token == 1;
   const int p = A.start[entry], lo = A.window > 0 ? max(0, p - A.window + 1) : 0;
   const int r_first = lo / AF_RANGE, r_last = p / AF_RANGE, range = r_first + (int)blockIdx.x;
-  pdl_wait();
-  if (!single || range > r_last) return;
+  if (!single || range > r_last) {
+    pdl_wait();
+    return;
+  }
   const int base = range * AF_RANGE, k_lo = max(0, lo - base), k_hi = min(AF_RANGE - 1, p - base);
   const int* table = A.table + (size_t)entry * A.table_width;
   const int chunks = d >> 2;
-  {
-    const int at = base + min(max(tid, k_lo), k_hi);
-    places[tid] = (((unsigned long long)table[at / A.page_size] * A.nkv + kvh) * A.page_size + at % A.page_size) * d;
+  if (tid < AF_RANGE) {
+    const int key = base + min(max(tid, k_lo), k_hi);
+    places[tid] = (((unsigned long long)table[key / A.page_size] * A.nkv + kvh) * A.page_size + key % A.page_size) * d;
   }
   __syncthreads();
+  auto fetch = [&](int begin, int end) {                        // 16-byte pieces of the range's keys and values
 #pragma unroll 4
-  for (int i = tid; i < (k_hi + 1) * chunks; i += AF_THREADS) {
-    const int k = i / chunks, c = i - k * chunks;
-    const unsigned long long off = places[k] + c * 4;
-    af_copy16(ks + k * pitch + c * 4, A.kpages + off, k >= k_lo);
-    af_copy16(vs + k * d + c * 4, A.vpages + off, k >= k_lo);
-  }
+    for (int i = begin + tid; i < end; i += AS_THREADS) {
+      const int k = i / chunks, c = i - k * chunks;
+      const unsigned long long off = places[k] + c * 4;
+      af_copy16(ks + k * pitch + c * 4, A.kpages + off, k >= k_lo);
+      af_copy16(vs + k * d + c * 4, A.vpages + off, k >= k_lo);
+    }
+  };
+  // earlier steps wrote all keys but the token's own, which comes from the kernel before this one
+  const int early = base + k_hi == p ? k_hi : k_hi + 1;
+  fetch(0, early * chunks);
+  pdl_wait();
+  fetch(early * chunks, (k_hi + 1) * chunks);
   af_commit();
   const float* q = A.qkv + (size_t)token * A.qkv_stride + (size_t)kvh * g * d;
   float* o = A.out + (size_t)token * A.nq * d + (size_t)kvh * g * d;
@@ -354,32 +369,32 @@ __global__ void __launch_bounds__(AF_THREADS) af32_single_kernel(const Af32Args 
   float* mine = part + (size_t)blockIdx.x * g * (d + 2);
   for (int h0 = 0; h0 < g; h0 += AF_HEADS) {
     const int nh = min(AF_HEADS, g - h0);
-    for (int i = tid; i < AF_HEADS * d; i += AF_THREADS) qs[i] = i < nh * d ? q[h0 * d + i] : 0.f;
+    for (int i = tid; i < AF_HEADS * d; i += AS_THREADS) qs[i] = i < nh * d ? q[h0 * d + i] : 0.f;
     af_wait<0>();
     __syncthreads();
-    {                                                           // a key a thread
-      f32x2 s[AF_HEADS];
+    {                                                           // a key and AS_PER heads a thread
+      f32x2 s[AS_PER];
 #pragma unroll
-      for (int h = 0; h < AF_HEADS; ++h) s[h] = 0;
-      if (tid >= k_lo && tid <= k_hi)
-#pragma unroll 4
+      for (int h = 0; h < AS_PER; ++h) s[h] = 0;
+      if (at >= k_lo && at <= k_hi)
+#pragma unroll 8
         for (int c = 0; c < chunks; ++c) {
-          const ulonglong2 k = af_lds2(ks + tid * pitch + c * 4);
+          const ulonglong2 k = af_lds2(ks + at * pitch + c * 4);
 #pragma unroll
-          for (int h = 0; h < AF_HEADS; ++h) {
-            const ulonglong2 x = af_lds2(qs + h * d + c * 4);
+          for (int h = 0; h < AS_PER; ++h) {
+            const ulonglong2 x = af_lds2(qs + (hq + h) * d + c * 4);
             s[h] = af_fma2(x.x, k.x, s[h]);
             s[h] = af_fma2(x.y, k.y, s[h]);
           }
         }
 #pragma unroll
-      for (int h = 0; h < AF_HEADS; ++h) {
+      for (int h = 0; h < AS_PER; ++h) {
         const float2 v = af_split(s[h]);
-        ps[h * AF_RANGE + tid] = tid >= k_lo && tid <= k_hi ? (v.x + v.y) * A.scale : -INFINITY;
+        ps[(hq + h) * AF_RANGE + at] = at >= k_lo && at <= k_hi ? (v.x + v.y) * A.scale : -INFINITY;
       }
     }
     __syncthreads();
-    for (int h = warp; h < nh; h += AF_THREADS / 32) {
+    for (int h = warp; h < nh; h += AS_THREADS / 32) {
       float* row = ps + h * AF_RANGE;
       float v[4];
 #pragma unroll
@@ -396,30 +411,32 @@ __global__ void __launch_bounds__(AF_THREADS) af32_single_kernel(const Af32Args 
       if (lane == 0) { stats[2 * h] = top; stats[2 * h + 1] = sum; }
     }
     __syncthreads();
-    if (tid < d) {                                              // a channel a thread
-      float a[AF_HEADS];
+    if (at < d) {                                               // a channel and AS_PER heads a thread
+      float a[AS_PER];
 #pragma unroll
-      for (int h = 0; h < AF_HEADS; ++h) a[h] = 0.f;
-      const float* v = vs + tid;
+      for (int h = 0; h < AS_PER; ++h) a[h] = 0.f;
+      const float* v = vs + at;
       int k = k_lo;
-      for (; k + 3 <= k_hi && k % 4 == 0; k += 4) {
+      for (; k % 4 && k <= k_hi; ++k)
+#pragma unroll
+        for (int h = 0; h < AS_PER; ++h) a[h] = fmaf(ps[(hq + h) * AF_RANGE + k], v[k * d], a[h]);
+#pragma unroll 4
+      for (; k + 3 <= k_hi; k += 4) {
         const float v0 = v[k * d], v1 = v[(k + 1) * d], v2 = v[(k + 2) * d], v3 = v[(k + 3) * d];
 #pragma unroll
-        for (int h = 0; h < AF_HEADS; ++h) {
-          const float4 e = *reinterpret_cast<const float4*>(ps + h * AF_RANGE + k);
+        for (int h = 0; h < AS_PER; ++h) {
+          const float4 e = *reinterpret_cast<const float4*>(ps + (hq + h) * AF_RANGE + k);
           a[h] = fmaf(e.w, v3, fmaf(e.z, v2, fmaf(e.y, v1, fmaf(e.x, v0, a[h]))));
         }
       }
-      for (; k <= k_hi; ++k) {
-        const float v0 = v[k * d];
+      for (; k <= k_hi; ++k)
 #pragma unroll
-        for (int h = 0; h < AF_HEADS; ++h) a[h] = fmaf(ps[h * AF_RANGE + k], v0, a[h]);
-      }
+        for (int h = 0; h < AS_PER; ++h) a[h] = fmaf(ps[(hq + h) * AF_RANGE + k], v[k * d], a[h]);
 #pragma unroll
-      for (int h = 0; h < AF_HEADS; ++h) {
-        if (h >= nh) continue;
-        if (ranges == 1) o[(h0 + h) * d + tid] = a[h] * (1.0f / stats[2 * h + 1]);
-        else mine[(size_t)(h0 + h) * (d + 2) + tid] = a[h];
+      for (int h = 0; h < AS_PER; ++h) {
+        if (hq + h >= nh) continue;
+        if (ranges == 1) o[(h0 + hq + h) * d + at] = a[h] * (1.0f / stats[2 * (hq + h) + 1]);
+        else mine[(size_t)(h0 + hq + h) * (d + 2) + at] = a[h];
       }
     }
     if (ranges > 1 && tid < 2 * nh) mine[(size_t)(h0 + (tid >> 1)) * (d + 2) + d + (tid & 1)] = stats[tid];
@@ -442,13 +459,13 @@ __global__ void __launch_bounds__(AF_THREADS) af32_single_kernel(const Af32Args 
   for (int h0 = 0; h0 < g; h0 += AF_HEADS) {
     const int nh = min(AF_HEADS, g - h0);
     float m = -INFINITY, l = 0.f;                                               // of head h0 + tid
-    float total[AF_HEADS];
+    float total[AS_PER];
 #pragma unroll
-    for (int h = 0; h < AF_HEADS; ++h) total[h] = 0.f;
+    for (int h = 0; h < AS_PER; ++h) total[h] = 0.f;
     for (int r0 = 0; r0 < ranges; r0 += AF_RANGE) {
       const int nr = min(AF_RANGE, ranges - r0);
       __syncthreads();
-      for (int i = tid; i < nh * nr; i += AF_THREADS) {
+      for (int i = tid; i < nh * nr; i += AS_THREADS) {
         const int h = i / nr, r = i - h * nr;
         factors[h * AF_RANGE + r] = __ldcg(reinterpret_cast<const float2*>(part + ((size_t)(r0 + r) * g + h0 + h) * (d + 2) + d));
       }
@@ -461,25 +478,25 @@ __global__ void __launch_bounds__(AF_THREADS) af32_single_kernel(const Af32Args 
           factors[tid * AF_RANGE + r] = make_float2(c1, c2);
         }
       __syncthreads();
-      if (tid < d)
+      if (at < d)
 #pragma unroll
-        for (int h = 0; h < AF_HEADS; ++h) {
-          if (h >= nh) continue;
-          const float* src = part + ((size_t)r0 * g + h0 + h) * (d + 2) + tid;
+        for (int h = 0; h < AS_PER; ++h) {
+          if (hq + h >= nh) continue;
+          const float* src = part + ((size_t)r0 * g + h0 + hq + h) * (d + 2) + at;
 #pragma unroll 8
           for (int r = 0; r < nr; ++r) {
             const float a = __ldcg(src + (size_t)r * g * (d + 2));
-            const float2 c = factors[h * AF_RANGE + r];
+            const float2 c = factors[(hq + h) * AF_RANGE + r];
             total[h] = c.y < 0.f ? total[h] : fmaf(total[h], c.x, a * c.y);
           }
         }
     }
     if (tid < nh) stats[tid] = l;
     __syncthreads();
-    if (tid < d)
+    if (at < d)
 #pragma unroll
-      for (int h = 0; h < AF_HEADS; ++h)
-        if (h < nh) o[(size_t)(h0 + h) * d + tid] = total[h] * (1.0f / stats[h]);
+      for (int h = 0; h < AS_PER; ++h)
+        if (hq + h < nh) o[(size_t)(h0 + hq + h) * d + at] = total[h] * (1.0f / stats[hq + h]);
   }
 }
 
@@ -515,7 +532,7 @@ Q25_EXPORT int q25_paged_attention_f32(const float* qkv, int qkv_stride, float* 
     const int smem = (AF_RANGE * (d + 4) + AF_RANGE * d + AF_HEADS * d + 2 * AF_HEADS * AF_RANGE + 2 * AF_HEADS) * 4;
     const cudaError_t e = cudaFuncSetAttribute(af32_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 150 * 1024);
     if (e != cudaSuccess) return (int)e;
-    launch(af32_single_kernel, dim3(ranges, nkv, entries), dim3(AF_THREADS), smem, s, A);
+    launch(af32_single_kernel, dim3(ranges, nkv, entries), dim3(AS_THREADS), smem, s, A);
   }
   return launch_status();
 }
