@@ -11,7 +11,7 @@
 // lanes of a warp can then work on different parts of K; and many short chains err less than one
 // long one.)
 //
-//   * up to 16 rows (decode steps): gemm_f32_rows_kernel, a stream of the weights;
+//   * up to 16 rows (decode steps), K and the row pitches multiples of 32: gemm_f32_rows_kernel, a stream of the weights;
 //   * more rows: gemm_f32_tile_kernel, bound by the FMA pipes;
 //   * operands TMA refuses (K or a row pitch not a multiple of 4, an unaligned base):
 //     gemm_f32_kernel, plain loads.
@@ -42,10 +42,14 @@ __device__ __forceinline__ void tma_2d(unsigned dst, const CUtensorMap* map, int
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void tma_2d_once(unsigned dst, const CUtensorMap* map, int x, int y, unsigned long long* bar,
+__device__ __forceinline__ void tma_3d(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
+               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+__device__ __forceinline__ void tma_3d_once(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar,
                                             unsigned long long policy) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;\n"
-               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "l"(policy) : "memory");
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;\n"
+               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "l"(policy) : "memory");
 }
 
 // ---- plain loads ----------------------------------------------------------------------------------------------------
@@ -115,20 +119,24 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 }
 
 // ---- up to 16 rows: a stream of the weights -------------------------------------------------------------------------
-// One persistent CTA per SM; its items are (group of 16 features, chunk of 512 k), one stage of the ring each: sixteen
-// TMA boxes of 16 rows x 32 floats (128-byte swizzle: eight lanes read eight rows of a column without a bank conflict)
-// and the chunk's columns of x.  A warp takes the items of one stage: lane = (pair of features p and p + 8, segment of
-// the chunk), so that 16 bytes of x serve two features, and leaves the segments' values in shared memory, where the last
-// warp adds them in order.  The producer starts the weights before it waits for the kernel before.
+// One persistent CTA per SM; its items are (group of 16 features, chunk of 512 k), one stage of the ring each, which two
+// copies fill: a box of 16 rows of W and one of the rows of x.  (The copy engine takes a request about every 90 cycles whatever
+// its size: as 16 boxes of 2 KB and four of x the stream ran at 5.2 TB/s.  22,016 features x 2,048 take 27 us for up to
+// two rows, 6.7 TB/s, 31 for four, 40 for eight and 71 for sixteen, where the reads of x out of shared memory count.)  K is seen as blocks of 32, and a row of W's box
+// holds 17 of them, the last one not used: with an odd number of 128-byte blocks a row, the 128-byte swizzle puts the
+// same block of eight rows into eight different bank groups.  A warp takes the items of one stage: lane = (pair of features p
+// and p + 8, segment of the chunk), so that 16 bytes of x serve two features, and leaves the segments' values in shared memory,
+// where the last warp adds them in order.  The producer starts the weights before it waits for the kernel before.
 // MT: rows of a lane; MG: warps that share a stage (rows 0 .. MT - 1 and MT ..).
 #define GR_ROWS 16
 #define GR_CHUNK 512
-#define GR_W_BYTES (GR_ROWS * GR_CHUNK * 4)
+#define GR_PITCH (17 * 128)                      // bytes between the rows of W in a stage
+#define GR_W_BYTES (GR_ROWS * GR_PITCH)
 
 template <int MT, int MG> struct RowsShape {
   static constexpr int MP = MT * MG;
   static constexpr int STAGE = GR_W_BYTES + MP * GR_CHUNK * 4;
-  static constexpr int STAGES = MP <= 2 ? 6 : MP == 4 ? 5 : MP == 8 ? 4 : 3;
+  static constexpr int STAGES = MP <= 4 ? 5 : MP == 8 ? 4 : 3;
   static constexpr int RED = 4 * GR_ROWS * MP;                  // floats of one slot of segment values
   static constexpr int WARPS = STAGES * MG;
   static constexpr int THREADS = (WARPS + 2) * 32;
@@ -170,17 +178,13 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       const unsigned long long once = l2_evict_first();
       bool ok = true;
       auto weights = [&](int item) {
-        const int s = item % S, g = (int)blockIdx.x + item / chunks * (int)gridDim.x, k0 = item % chunks * GR_CHUNK;
-        const int boxes = min(GR_CHUNK / 32, (K - k0 + 31) / 32), segs = min(4, (K - k0 + GF_SEG - 1) / GF_SEG);
-        const unsigned st = smem_u32(smem + s * Shape::STAGE);
-        mbar_expect_tx(full + s, (unsigned)(boxes * GR_ROWS * 128 + segs * MP * GF_SEG * 4));
-        for (int b = 0; b < boxes; ++b)
-          tma_2d_once(st + b * (GR_ROWS * 128), &map_w, k0 + b * 32, g * GR_ROWS, full + s, once);
+        const int s = item % S, g = (int)blockIdx.x + item / chunks * (int)gridDim.x, block = item % chunks * (GR_CHUNK / 32);
+        mbar_expect_tx(full + s, Shape::STAGE);
+        tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, block, g * GR_ROWS, full + s, once);
       };
       auto rows = [&](int item) {
-        const int s = item % S, k0 = item % chunks * GR_CHUNK, segs = min(4, (K - k0 + GF_SEG - 1) / GF_SEG);
-        const unsigned st = smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES;
-        for (int g = 0; g < segs; ++g) tma_2d(st + g * (MP * GF_SEG * 4), &map_x, k0 + g * GF_SEG, 0, full + s);
+        const int s = item % S, block = item % chunks * (GR_CHUNK / 32);
+        tma_3d(smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES, &map_x, 0, block, 0, full + s);
       };
       const int ahead = min(S, items);
       for (int i = 0; i < ahead; ++i) weights(i);
@@ -236,8 +240,8 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   const int s = warp / MG, mg = warp % MG, p = lane & 7, seg = lane >> 3;
   bool ok = true;
   unsigned parity = 0;
-  const unsigned wa = smem_u32(smem + s * Shape::STAGE) + seg * (4 * GR_ROWS * 128) + p * 128;
-  const unsigned xa = smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES + seg * (MP * GF_SEG * 4) + mg * MT * (GF_SEG * 4);
+  const unsigned wa = smem_u32(smem + s * Shape::STAGE) + p * GR_PITCH + seg * 512;
+  const unsigned xa = smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES + mg * MT * (GR_CHUNK * 4) + seg * 512;
   for (int i = s; i < items; i += S, parity ^= 1) {
     const int left = K - i % chunks * GR_CHUNK - seg * GF_SEG, blocks = min(4, (left + 31) / 32);        // may be <= 0
     f32x2 acc[2][MT];
@@ -250,11 +254,11 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     for (int b = 0; b < blocks; ++b) {
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        const unsigned at = wa + b * (GR_ROWS * 128) + ((c ^ p) << 4);
-        const ulonglong2 w0 = lds_pair(at), w1 = lds_pair(at + 8 * 128);
+        const unsigned at = wa + b * 128 + ((c ^ ((p + seg * 4 + b) & 7)) << 4);
+        const ulonglong2 w0 = lds_pair(at), w1 = lds_pair(at + 8 * GR_PITCH);
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-          const ulonglong2 x = lds_pair(xa + m * (GF_SEG * 4) + b * 128 + c * 16);
+          const ulonglong2 x = lds_pair(xa + m * (GR_CHUNK * 4) + b * 128 + c * 16);
           acc[0][m] = fma2(w0.x, x.x, acc[0][m]);
           acc[1][m] = fma2(w1.x, x.x, acc[1][m]);
           acc[0][m] = fma2(w0.y, x.y, acc[0][m]);
@@ -512,21 +516,38 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// A [rows, K] float matrix with row pitch ld, boxes of box_rows x box_k (swizzled when a box row is 128 bytes).
-static bool make_map_f32(CUtensorMap* map, const float* base, int rows, int K, int ld, int box_rows, int box_k) {
+static EncodeTiledFn encode_tiled() {
   static EncodeTiledFn enc = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
     return reinterpret_cast<EncodeTiledFn>(p);
   }();
+  return enc;
+}
+
+// A [rows, K] float matrix with row pitch ld, boxes of box_rows x 32 in the 128-byte swizzle.
+static bool make_map_f32(CUtensorMap* map, const float* base, int rows, int K, int ld, int box_rows) {
+  EncodeTiledFn enc = encode_tiled();
   if (!enc) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  const cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
+  const cuuint32_t box[2] = {32, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             box_k == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The same with K as blocks of 32 (K and ld multiples of 32): boxes of box_rows x box_blocks blocks.
+static bool make_blocks_f32(CUtensorMap* map, const float* base, int rows, int K, int ld, int box_rows, int box_blocks, bool swizzle) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint64_t dims[3] = {32, (cuuint64_t)(K / 32), (cuuint64_t)rows};
+  const cuuint64_t strides[2] = {128, (cuuint64_t)ld * 4};
+  const cuuint32_t box[3] = {32, (cuuint32_t)box_blocks, (cuuint32_t)box_rows};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -535,7 +556,7 @@ static int launch_rows(const float* A, const float* W, const float* bias, float*
                        int* err, cudaStream_t s) {
   using Shape = RowsShape<MT, MG>;
   CUtensorMap mx, mw;
-  if (!make_map_f32(&mx, A, M, K, lda, Shape::MP, GF_SEG) || !make_map_f32(&mw, W, N, K, ldw, GR_ROWS, 32)) return (int)cudaErrorInvalidValue;
+  if (!make_blocks_f32(&mx, A, M, K, lda, Shape::MP, GR_CHUNK / 32, false) || !make_blocks_f32(&mw, W, N, K, ldw, GR_ROWS, 17, true)) return (int)cudaErrorInvalidValue;
   const cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<MT, MG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
   if (e != cudaSuccess) return (int)e;
   const int sms = device_sm_count(), groups = (N + GR_ROWS - 1) / GR_ROWS;
@@ -557,7 +578,7 @@ static int launch_tile(const float* A, const float* W, const float* bias, float*
                        int* err, long long per_sm, cudaStream_t s) {
   const int SMEM = smem_for(1024 + GT_STAGES * (WM + WN) * 32 * 128 + GT_STAGES * 16, per_sm);
   CUtensorMap ma, mw;
-  if (!make_map_f32(&ma, A, M, K, lda, WM * 32, 32) || !make_map_f32(&mw, W, N, K, ldw, WN * 32, 32)) return (int)cudaErrorInvalidValue;
+  if (!make_map_f32(&ma, A, M, K, lda, WM * 32) || !make_map_f32(&mw, W, N, K, ldw, WN * 32)) return (int)cudaErrorInvalidValue;
   const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<WM, WN, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   if (e != cudaSuccess) return (int)e;
   launch(gemm_f32_tile_kernel<WM, WN, CTAS>, dim3((M + WM * 32 - 1) / (WM * 32), (N + WN * 32 - 1) / (WN * 32)), dim3(WM * WN * 32), SMEM, s,
@@ -585,11 +606,13 @@ Q25_EXPORT int q25_gemm_f32(const float* A, const float* W, const float* bias, f
     }
     return launch_status();
   }
-  if (M == 1) return launch_rows<1, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
-  if (M == 2) return launch_rows<2, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
-  if (M <= 4) return launch_rows<4, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
-  if (M <= 8) return launch_rows<8, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
-  if (M <= 16) return launch_rows<8, 2>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
+  if (M <= 16 && K % 32 == 0 && lda % 32 == 0 && ldw % 32 == 0) {
+    if (M == 1) return launch_rows<1, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
+    if (M == 2) return launch_rows<2, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
+    if (M <= 4) return launch_rows<4, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
+    if (M <= 8) return launch_rows<8, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
+    return launch_rows<8, 2>(A, W, bias, C, M, N, K, lda, ldw, ldc, err, s);
+  }
   // Which tile ends first: q CTAs on the fullest SM, each an area of outputs, at the FMAs a clock that an SM was measured to
   // do with one, two or more such CTAs (of 128; 1,500 rows x 22,016 features: 45 TFLOP/s with 64 x 64, 41 with 32 x 32, but
   // 64 rows x 2,048 features, K 11,008: 432 against 112 us, and 1,500 x 2,048: 340 against 321 us).
@@ -601,7 +624,7 @@ Q25_EXPORT int q25_gemm_f32(const float* A, const float* W, const float* bias, f
   if (t32 < t64 && (N + 31) / 32 <= 65535) {
     const int stages = q32 == 1 ? 4 : 2;
     CUtensorMap ma, mw;
-    if (!make_map_f32(&ma, A, M, K, lda, 32, 32) || !make_map_f32(&mw, W, N, K, ldw, 32, 32)) return (int)cudaErrorInvalidValue;
+    if (!make_map_f32(&ma, A, M, K, lda, 32) || !make_map_f32(&mw, W, N, K, ldw, 32)) return (int)cudaErrorInvalidValue;
     const cudaError_t e = cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return (int)e;
     launch(gemm_f32_split_kernel, dim3((M + 31) / 32, (N + 31) / 32), dim3(GS_WARPS * 32), smem_for(GS_SMEM(stages), q32), s, ma, mw, bias, C, M, N, K, ldc,

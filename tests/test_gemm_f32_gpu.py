@@ -9,7 +9,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 #  rows, features, K, pitch of the rows beyond K
-CASES = [(1, 17, 4, 0), (2, 16, 36, 0), (3, 300, 512, 0), (5, 33, 516, 0), (9, 64, 1028, 12), (16, 2400, 640, 0), (4, 16, 11008, 0),
+CASES = [(1, 17, 4, 0), (2, 16, 36, 0), (3, 300, 512, 0), (5, 33, 516, 0), (9, 64, 1028, 12), (16, 2400, 640, 0), (4, 16, 11008, 0), (2, 40, 32, 32), (7, 50, 544, 0), (12, 5000, 96, 64),
          (17, 31, 132, 0), (64, 2048, 2052, 0), (33, 65, 4096, 4), (256, 130, 100, 0),                      # warps side by side in K
          (640, 1990, 260, 0), (700, 4100, 128, 8),                                                          # tiles of 64 x 64
          (3, 100, 257, 0), (70, 70, 64, 1)]                                                                  # plain loads
