@@ -1,8 +1,8 @@
 // Causal attention over the paged cache for a batch of (request, run of tokens): the general
 // kernel.  It takes any head size that is a multiple of 16 up to 256, any number of heads and
 // groups, any page size, a window or none, float or bfloat16, and any mixture of run lengths.
-// It is the only attention of the 32-bit path and the fallback of the serving path for sizes the
-// tensor-core kernels refuse.
+// It takes what the other kernels refuse: in 32 bits heads above 128 channels (attention_f32.cu has the
+// others), on the serving path sizes the tensor-core kernels do not take.
 //
 // Formula (reference: zhangjianbang-nb/qwen25vl-lite): S = (q . k^T) * D^-1/2; the query at
 // absolute index a = computed + i sees keys j <= a; softmax over keys; o = P v; query head h
