@@ -17,6 +17,7 @@
 //     gemm_f32_kernel, plain loads.
 #include "common.cuh"
 #include "f32x2.cuh"
+#include "gemm_f32x3.cuh"
 #include "tensor_map.cuh"
 
 #define GF_SEG 128                               // k of one segment
@@ -565,9 +566,11 @@ static int launch_tile(const float* A, const float* W, const float* bias, float*
 }
 
 // The zero padding of the K tail adds fma(0, 0, acc) = acc, which leaves the chains unchanged.
-// fixed: no kernel writes W, so it may be fetched before the kernel ahead has ended.  err: device int that gets a code if a bounded
-// wait gave up.
-Q25_EXPORT int q25_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda,
+// fixed: no kernel writes W, so it may be fetched before the kernel ahead has ended.  scratch: what q25_gemm_f32_scratch says, 16-byte
+// aligned, for products that the tensor cores take, but not for up to F32X3_FEW rows that are aligned to 16 bytes.  err: device int that
+// gets a code if a bounded wait gave up.
+Q25_EXPORT long long q25_gemm_f32_scratch(int M, int N, int K) { return M > 0 && N > 0 && f32x3_takes(K) ? (long long)f32x3_scratch(M, N, K) : 0; }
+Q25_EXPORT int q25_gemm_f32(const float* A, const float* W, const float* bias, float* C, void* scratch, int M, int N, int K, int lda,
                             int ldw, int ldc, int fixed, int* err, void* stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || !err) return (int)cudaErrorInvalidValue;
@@ -575,6 +578,12 @@ Q25_EXPORT int q25_gemm_f32(const float* A, const float* W, const float* bias, f
   const bool early = fixed != 0;
   if (M == 1) lda = K;                             // a single row's pitch says nothing
   if (N == 1) ldw = K;
+  if (f32x3_takes(K) && ldw % 4 == 0 && ldw >= K && !((uintptr_t)W & 15)) {
+    if (M <= F32X3_FEW && lda % 4 == 0 && lda >= K && !((uintptr_t)A & 15))
+      return launch_f32x3_few(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
+    if (!scratch || ((uintptr_t)scratch & 15)) return (int)cudaErrorInvalidValue;
+    return launch_f32x3_many(A, W, bias, C, scratch, M, N, K, lda, ldw, ldc, early, err, s);
+  }
   const bool tma = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && lda >= K && ldw >= K && !((uintptr_t)A & 15) && !((uintptr_t)W & 15);
   // Few steps of K: the other kernels' start counts for more than their loads (a row of K 16: 2.5 against 3.2 us; and for the many
   // CTAs of a large vocabulary, 152,064 features: K 48 and up to four rows 25 against 34, K 64 and eight 35 against 52, K 128

@@ -1,0 +1,754 @@
+// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) of 32-bit operands on the tensor cores, no less precise than by 32-bit FMAs.
+//
+// A 32-bit number is the sum of three bfloat16 numbers, hi + mid + lo: hi is the number rounded, mid what hi leaves, rounded,
+// lo the rest; 8 bits of the mantissa each, so nothing is lost.  Of the nine products of two such sums the six largest are taken;
+// the others (mid lo, lo mid, lo lo) are below 2^-24 of the product.  bfloat16 products are exact in 32 bits, what remains is how
+// they are added.  The tensor core cuts bits off where FMA rounds, so it adds no more than 32 k (two instructions of 16 k for
+// each of the six, the small ones first); the values of these chunks are added by ordinary 32-bit additions.  For every
+// output element, whatever kernel computes it:
+//
+//   chunk   32 k: lo.hi, hi.lo, mid.mid, mid.hi, hi.mid, hi.hi (weight . row), 16 k and then the next 16 k of each, into one
+//           accumulator that begins at 0;
+//   block   256 k: its chunks' values, added in order;
+//   result  the blocks' values, added in order; then + bias.
+//
+// The order depends on nothing but K, so a token's result is bit for bit the same whether it is computed alone, in a portion or in a
+// large batch: mma.sync and tcgen05.mma give the same bits for the same 16 k (test_gemm_f32x3_gpu.py holds them to it).
+// A result that is not finite (an infinite or not-a-number operand has no three parts; a part may round up to infinity) is
+// computed again by plain FMA.
+//
+//   * up to 16 rows (decode steps): f3_rows_kernel, a stream of the weights, mma.sync;
+//   * more rows: f3_parts_kernel cuts A into its three parts, f3_tile_kernel multiplies, tcgen05; where its tiles are too few
+//     for the SMs, a tile's blocks go to several CTAs and f3_sum_kernel adds them.
+#include "f32x2.cuh"
+#include "gemm_f32x3.cuh"
+#include "tcgen05.cuh"
+#include "tensor_map.cuh"
+
+#define F3_CHUNK 32
+#define F3_BLOCK 256
+#define F3_BLOCK_CHUNKS (F3_BLOCK / F3_CHUNK)
+
+// The parts of two neighbours, packed as the tensor core reads them (the first in the low half).
+__device__ __forceinline__ unsigned f3_pack(float lo, float hi) {
+  unsigned r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ f32x2 f3_less(f32x2 x, unsigned part) {       // what a part leaves
+  f32x2 r;
+  asm("{\n .reg .b32 a, b;\n .reg .b64 p;\n shl.b32 a, %2, 16;\n and.b32 b, %2, 0xffff0000;\n mov.b64 p, {a, b};\n"
+      " sub.rn.f32x2 %0, %1, p;\n}\n" : "=l"(r) : "l"(x), "r"(part));
+  return r;
+}
+__device__ __forceinline__ void f3_split(f32x2 x, unsigned& hi, unsigned& mid, unsigned& lo) {
+  float2 v = split2(x);
+  hi = f3_pack(v.x, v.y);
+  x = f3_less(x, hi);
+  v = split2(x);
+  mid = f3_pack(v.x, v.y);
+  x = f3_less(x, mid);
+  v = split2(x);
+  lo = f3_pack(v.x, v.y);
+}
+
+__device__ __forceinline__ ulonglong2 f3_lds(unsigned addr) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];\n" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ bool f3_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+// A result by plain FMA, in the order of gemm_f32.cu.
+__device__ __noinline__ float f3_plain(const float* __restrict__ a, const float* __restrict__ w, int K) {
+  float total = 0.f;
+  for (int k0 = 0; k0 < K; k0 += 128) {
+    float even = 0.f, odd = 0.f;
+    for (int k = k0; k < min(K, k0 + 128); k += 2) {
+      even = fmaf(a[k], w[k], even);
+      odd = fmaf(a[k + 1], w[k + 1], odd);
+    }
+    total += even + odd;
+  }
+  return total;
+}
+// The results of rows m .. end of a feature that are not finite, computed again.
+__device__ __noinline__ void f3_again(const float* A, const float* W, float* C, int m, int end, int n, int K, int lda, int ldw, int ldc, float more) {
+  for (; m < end; ++m) {
+    float* c = C + (size_t)m * ldc + n;
+    if (!f3_finite(*c)) *c = f3_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K) + more;
+  }
+}
+
+__device__ __forceinline__ void f3_tma_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void f3_tma_3d(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
+               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+__device__ __forceinline__ void f3_tma_3d_once(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar,
+                                               unsigned long long policy) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;\n"
+               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "l"(policy) : "memory");
+}
+
+// ---- up to 16 rows: a stream of the weights -------------------------------------------------------------------------
+// One persistent CTA per SM; its items are (group of 16 features, 512 k), one stage of the ring each, which two copies fill: a
+// box of 16 rows of W and one of the rows of x (the copy engine takes a request about every 90 cycles whatever its size).  K is
+// seen as lines of 32; a row of W's box holds 17 of them, the last one not used, so that the 128-byte swizzle puts the same
+// line of eight rows into eight different bank groups.  Four warps share a stage, half a block each: the weights are
+// the 16-row side of mma.sync m16n8k16, the rows of x its 8 columns (two such tiles for 9 to 16 rows), and a thread's 16 bytes
+// of a row fill its four k slots (the sum over 16 k has no order).  A chunk's 12 MMAs wait for one another, so it takes many
+// warps to keep up with the copies.  The warp of a block's second half adds its chunks to the first half's sum, in shared
+// memory, where one more warp adds the blocks.
+#define F3R_FEATURES 16
+#define F3R_K 512
+#define F3R_PITCH (17 * 128)                     // bytes between the rows of W in a stage
+#define F3R_W_BYTES (F3R_FEATURES * F3R_PITCH)
+
+template <int MP> struct F3Rows {                // MP: rows of x in a stage
+  static constexpr int TILES = MP > 8 ? 2 : 1;
+  static constexpr int STAGE = F3R_W_BYTES + MP * F3R_K * 4;
+  static constexpr int STAGES = MP <= 4 ? 5 : MP == 8 ? 4 : 3;
+  static constexpr int RED = 2 * F3R_FEATURES * MP;             // floats of one slot of block values
+  static constexpr int WARPS = STAGES * 4;
+  static constexpr int THREADS = (WARPS + 2) * 32;
+  static constexpr int SMEM = 1024 + STAGES * (STAGE + RED * 4) + STAGES * 4 * 8;
+};
+
+__device__ __forceinline__ void f3_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+template <int MP>
+__global__ void __launch_bounds__(F3Rows<MP>::THREADS, 1)
+f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const float* __restrict__ A,
+               const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K, int lda, int ldw,
+               int ldc, bool early, int* err) {
+  using Shape = F3Rows<MP>;
+  constexpr int S = Shape::STAGES, TILES = Shape::TILES;
+  extern __shared__ unsigned char f3_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)f3_raw + 1023) & ~(uintptr_t)1023);
+  float* red = reinterpret_cast<float*>(smem + S * Shape::STAGE);
+  unsigned long long* full = reinterpret_cast<unsigned long long*>(red + S * Shape::RED);
+  unsigned long long* empty = full + S;
+  unsigned long long* red_full = empty + S;
+  unsigned long long* red_empty = red_full + S;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int spans = (K + F3R_K - 1) / F3R_K, groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
+  const int items = ((groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * spans;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 4);
+      mbar_init(red_full + s, 2);
+      mbar_init(red_empty + s, 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+  pdl_trigger();
+
+  if (warp == Shape::WARPS) {
+    // ---- producer ----
+    if (lane == 0) {
+      const unsigned long long once = l2_evict_first();
+      bool ok = true;
+      auto weights = [&](int item) {
+        const int s = item % S, g = (int)blockIdx.x + item / spans * (int)gridDim.x, line = item % spans * (F3R_K / 32);
+        mbar_expect_tx(full + s, Shape::STAGE);
+        f3_tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, line, g * F3R_FEATURES, full + s, once);
+      };
+      auto rows = [&](int item) {
+        const int s = item % S, line = item % spans * (F3R_K / 32);
+        f3_tma_3d(smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES, &map_x, 0, line, 0, full + s);
+      };
+      const int ahead = min(S, items);
+      if (!early) pdl_wait();
+      for (int i = 0; i < ahead; ++i) weights(i);
+      pdl_wait();
+      for (int i = 0; i < ahead; ++i) rows(i);
+      for (int i = ahead; i < items; ++i) {
+        if (ok) {
+          ok = mbar_wait(empty + i % S, (unsigned)(i / S - 1) & 1);
+          if (!ok) { atomicExch(err, 51); break; }               // nobody reads what was not asked for: the readers give up too
+        }
+        weights(i);
+        rows(i);
+      }
+    }
+    return;
+  }
+  if (warp == Shape::WARPS + 1) {
+    // ---- the blocks' values, added in order ----
+    constexpr int V = (F3R_FEATURES * MP + 31) / 32;
+    pdl_wait();                                                  // the kernel before may still read what this one overwrites
+    bool ok = true;
+    float total[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) total[v] = 0.f;
+    for (int i = 0; i < items; ++i) {
+      const int s = i % S;
+      if (ok) {
+        ok = mbar_wait(red_full + s, (unsigned)(i / S) & 1);
+        if (!ok && lane == 0) atomicExch(err, 52);
+      }
+      const float* slot = red + s * Shape::RED;
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          if (V * 32 == F3R_FEATURES * MP || lane < F3R_FEATURES * MP) total[v] += slot[q * (F3R_FEATURES * MP) + v * 32 + lane];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(red_empty + s);
+      if (i % spans == spans - 1) {
+        const int n = ((int)blockIdx.x + i / spans * (int)gridDim.x) * F3R_FEATURES + (lane & 15);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const int m = v * 2 + (lane >> 4);
+          if (m < M && n < N) {
+            if (!f3_finite(total[v])) total[v] = f3_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+            C[(size_t)m * ldc + n] = total[v] + (bias ? bias[n] : 0.f);
+          }
+          total[v] = 0.f;
+        }
+      }
+    }
+    return;
+  }
+
+  // ---- four warps, one stage ----
+  // MMA row g of the 16 is feature (g mod 2) * 4 + g / 2 of the group, and row g + 8 that + 8: the two rows whose 64 bytes a warp reads
+  // together then lie in different halves of the banks.
+  const int s = warp >> 2, block = (warp >> 1) & 1, half = warp & 1, g = lane >> 2, t = lane & 3, f = (g & 1) * 4 + (g >> 1);
+  const int pair = 1 + (warp >> 1);                              // the named barrier of a block's two warps
+  bool ok = true;
+  unsigned parity = 0;
+  const unsigned line0 = (block * F3_BLOCK_CHUNKS + half * 4) * 128;
+  const unsigned wa = smem_u32(smem + s * Shape::STAGE) + f * F3R_PITCH + line0;
+  const unsigned xa = smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES + (g & (MP < 8 ? MP - 1 : 7)) * (F3R_K * 4) + line0 + t * 16;
+  float* slot = red + s * Shape::RED + block * (F3R_FEATURES * MP) + f;
+  for (int i = s; i < items; i += S, parity ^= 1) {
+    const int left = (K - i % spans * F3R_K - block * F3_BLOCK) / F3_CHUNK - half * 4;        // chunks; may be <= 0
+    float v[4][TILES][4];
+    if (ok) {
+      ok = mbar_wait(full + s, parity);
+      if (!ok && lane == 0) atomicExch(err, 53);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+#pragma unroll
+      for (int n = 0; n < TILES; ++n) v[c][n][0] = v[c][n][1] = v[c][n][2] = v[c][n][3] = 0.f;
+      if (c >= left) continue;
+      unsigned a[2][3][4], b[TILES][2][3][2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const unsigned at = wa + c * 128 + (((h * 4 + t) ^ ((f + half * 4 + c) & 7)) << 4);        // a block's 8 lines are a whole turn of the swizzle
+        const ulonglong2 w0 = f3_lds(at), w1 = f3_lds(at + 8 * F3R_PITCH);
+        f3_split(w0.x, a[h][0][0], a[h][1][0], a[h][2][0]);
+        f3_split(w1.x, a[h][0][1], a[h][1][1], a[h][2][1]);
+        f3_split(w0.y, a[h][0][2], a[h][1][2], a[h][2][2]);
+        f3_split(w1.y, a[h][0][3], a[h][1][3], a[h][2][3]);
+#pragma unroll
+        for (int n = 0; n < TILES; ++n) {
+          const ulonglong2 x = f3_lds(xa + n * (8 * F3R_K * 4) + c * 128 + h * 64);
+          f3_split(x.x, b[n][h][0][0], b[n][h][1][0], b[n][h][2][0]);
+          f3_split(x.y, b[n][h][0][1], b[n][h][1][1], b[n][h][2][1]);
+        }
+      }
+      constexpr int wp[6] = {2, 0, 1, 1, 0, 0}, xp[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+      for (int p = 0; p < 6; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int n = 0; n < TILES; ++n) f3_mma(v[c][n], a[h][wp[p]], b[n][h][xp[p]]);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + s);
+    if (half == 0) {
+      if (i >= S && ok) {
+        ok = mbar_wait(red_empty + s, parity ^ 1);
+        if (!ok && lane == 0) atomicExch(err, 54);
+      }
+      __syncwarp();
+    } else {
+      asm volatile("bar.sync %0, 64;\n" ::"r"(pair) : "memory");
+    }
+#pragma unroll
+    for (int n = 0; n < TILES; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int m = n * 8 + 2 * t + (e & 1);
+        float* at = slot + m * F3R_FEATURES + 8 * (e >> 1);
+        if (m >= MP) continue;
+        float sum = half == 0 ? v[0][n][e] : *at + v[0][n][e];
+        sum += v[1][n][e];
+        sum += v[2][n][e];
+        *at = sum + v[3][n][e];
+      }
+    if (half == 0) {
+      asm volatile("bar.arrive %0, 64;\n" ::"r"(pair) : "memory");
+    } else {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(red_full + s);
+    }
+  }
+}
+
+// ---- more rows: the parts of A --------------------------------------------------------------------------------------
+// parts[3][M][K]: 10 bytes a value pass through memory, once; f3_tile_kernel then reads A's tiles as the tensor core wants them
+// (a tile of A is read by N / 128 CTAs, each of which would have to cut it up again).
+__global__ void __launch_bounds__(256)
+f3_parts_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, int K, int lda, bool aligned) {
+  pdl_trigger();
+  pdl_wait();
+  const size_t eighths = (size_t)M * (K / 8);
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < eighths; i += (size_t)gridDim.x * 256) {
+    const size_t row = i / (K / 8);
+    const float* src = A + row * lda + (i - row * (K / 8)) * 8;
+    float v[8];
+    if (aligned) {
+      const float4 p = __ldcg(reinterpret_cast<const float4*>(src)), q = __ldcg(reinterpret_cast<const float4*>(src) + 1);
+      v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w;
+      v[4] = q.x; v[5] = q.y; v[6] = q.z; v[7] = q.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __ldcg(src + j);
+    }
+    unsigned p[3][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) f3_split(pair2(v[2 * j], v[2 * j + 1]), p[0][j], p[1][j], p[2][j]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) parts[q * eighths + i] = make_uint4(p[q][0], p[q][1], p[q][2], p[q][3]);
+  }
+}
+
+// ---- more rows: tiles of 128 features x BN rows ---------------------------------------------------------------------
+// One CTA per SM.  The features are the 128 lanes of tensor memory, the rows of A its columns.  An instruction of both operands
+// from shared memory would read 8 KB in 64 cycles (BN 128), all of its bandwidth, before W is even cut up.  So W's parts go to tensor
+// memory: converter warps take 32 k of W's 128 rows from the ring (32-bit, 16 KB), a thread a row, and store the three parts as the A
+// operand (48 columns, two such stages); A's parts come by TMA ready to be read (64 k a stage).
+// The MMA warp leaves the value of each chunk of 32 k in one of two accumulators of BN columns; the drain warps add it in
+// registers, and a block's value to the result so far, which lies in tensor memory as well (BN columns).
+// With splits > 1 a tile's blocks are cut into that many ranges, a CTA each, and every block's value goes to its plane [M][N] of
+// `planes`, for f3_sum_kernel.
+// Warps: 4 drain a tile of up to 64 rows, 8 a wider one (half of its columns each, which is what their registers hold); then 4
+// converters, or 8 where a chunk's MMAs leave less time (the second four take the odd chunks); a producer for W, which runs ahead
+// of the kernel before, one for A's parts, and the MMA warp.
+template <int BN> struct F3Tile {
+  static constexpr int XSTAGE = 3 * BN * 128, WSTAGE = 128 * 128;
+  static constexpr int XS = BN >= 96 ? 3 : 4;
+  static constexpr int SETS = BN >= 96 ? 1 : 2;                 // of four converter warps
+  static constexpr int ROOM = (208 * 1024 - XS * XSTAGE) / WSTAGE;
+  static constexpr int WS = ROOM > 8 ? 8 : ROOM / SETS * SETS;  // a stage always serves the same set
+  static constexpr int DRAINS = BN >= 96 ? 8 : 4, WIDTH = BN * 4 / DRAINS;         // columns a drain warp has
+  static constexpr int STEP = WIDTH % 32 == 0 ? 32 : 16;                           // and takes at a time
+  static constexpr int WARPS = DRAINS + 4 * SETS + 3;
+  static constexpr int THREADS = WARPS * 32;
+  static constexpr int TOTAL = 2 * BN, PARTS = 3 * BN;          // columns: accumulators at 0 and BN, the result so far, W's parts
+  static constexpr int SMEM = 1024 + XS * XSTAGE + WS * WSTAGE + 512;
+  static_assert(3 * BN + 96 <= 512 && WS % SETS == 0, "tensor memory; stages");
+};
+
+// 16 words into this thread's lane of tensor memory; 16 or 32 floats out of it and back.
+__device__ __forceinline__ void f3_st16(unsigned taddr, const unsigned (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void f3_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void f3_ld(unsigned taddr, float (&v)[32]) { tc5_ld32(taddr, v); }
+__device__ __forceinline__ void f3_ld(unsigned taddr, float (&v)[16]) {
+  unsigned r[16];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                 "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void f3_st(unsigned taddr, const float (&v)[32]) { tc5_st32(taddr, v); }
+__device__ __forceinline__ void f3_st(unsigned taddr, const float (&v)[16]) {
+  unsigned r[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(v[i]);
+  f3_st16(taddr, r);
+  f3_st_wait();
+}
+__device__ __forceinline__ bool f3_elect() {
+  unsigned e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+  return e != 0;
+}
+__device__ constexpr unsigned f3_idesc(int n) {                  // bf16 x bf16 -> f32, M 128, N n, both operands K-major
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
+}
+
+template <int BN>
+__global__ void __launch_bounds__(F3Tile<BN>::THREADS, 1)
+f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_w, const float* __restrict__ A,
+               const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, float* __restrict__ planes, int splits, int M,
+               int N, int K, int lda, int ldw, int ldc, bool early, int* err) {
+  using Shape = F3Tile<BN>;
+  constexpr int XS = Shape::XS, WS = Shape::WS, SETS = Shape::SETS;
+  extern __shared__ unsigned char f3_raw[];
+  unsigned char* xring = reinterpret_cast<unsigned char*>(((uintptr_t)f3_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* wring = xring + XS * Shape::XSTAGE;
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(wring + WS * Shape::WSTAGE);
+  unsigned long long *w_full = bars, *w_empty = w_full + WS, *x_full = w_empty + WS, *x_empty = x_full + XS;
+  // of each of the two buffers (a stage of W's parts and an accumulator): both are free for the MMAs; these have ended
+  unsigned long long *ready = x_empty + XS, *done = ready + 2;
+  unsigned* tmem_at = reinterpret_cast<unsigned*>(done + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int W_WARP = Shape::DRAINS + 4 * SETS, X_WARP = W_WARP + 1, MMA_WARP = W_WARP + 2;
+  const int row_tiles = (M + BN - 1) / BN, tiles = row_tiles * ((N + 127) / 128);
+  // this CTA's tiles, and the chunks of K that it takes of each (whole blocks; a split tile's CTAs have one tile)
+  const int first_tile = (int)blockIdx.x / splits, part = (int)blockIdx.x % splits, step = (int)gridDim.x;
+  const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK;
+  const int c_begin = (int)((long long)blocks * part / splits) * F3_BLOCK_CHUNKS;
+  const int c_end = min(K / F3_CHUNK, (int)((long long)blocks * (part + 1) / splits) * F3_BLOCK_CHUNKS), chunks = c_end - c_begin;
+  const int mine = (tiles - first_tile + step - 1) / step * chunks;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < WS; ++s) { mbar_init(w_full + s, 1); mbar_init(w_empty + s, 4); }
+    for (int s = 0; s < XS; ++s) { mbar_init(x_full + s, 1); mbar_init(x_empty + s, 1); }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(ready + b, 4 + Shape::DRAINS);
+      mbar_init(done + b, 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+  pdl_trigger();
+  auto load_w = [&](int it) {
+    const int tile = first_tile + it / chunks * step, s = it % WS;
+    mbar_expect_tx(w_full + s, Shape::WSTAGE);
+    f3_tma_2d(smem_u32(wring + s * Shape::WSTAGE), &map_w, (c_begin + it % chunks) * F3_CHUNK, tile / row_tiles * 128, w_full + s);
+  };
+  const int ahead = min(WS, mine);
+  if (early && warp == W_WARP && lane == 0)
+    for (int it = 0; it < ahead; ++it) load_w(it);
+  // A's parts come from the kernel before this one, and tensor memory is asked for only when that has gone (gemm_tcgen05.cu)
+  pdl_wait();
+  if (!early && warp == W_WARP && lane == 0)
+    for (int it = 0; it < ahead; ++it) load_w(it);
+  __syncwarp();
+  if (warp == MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tmem_at)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  tc5_fence_before();
+  __syncthreads();
+  tc5_fence_after();
+  const unsigned tmem = *tmem_at;
+  bool ok = true;
+
+  if (warp == W_WARP) {
+    if (lane == 0)
+      for (int it = ahead; it < mine; ++it) {
+        if (!mbar_wait(w_empty + it % WS, (unsigned)(it / WS - 1) & 1)) { atomicExch(err, 55); break; }
+        load_w(it);
+      }
+  } else if (warp == X_WARP) {
+    if (lane == 0) {
+      int xt = 0;
+      for (int tile = first_tile; tile < tiles && ok; tile += step)
+        for (int c = c_begin; c < c_end; c += 2, ++xt) {
+          const int s = xt % XS;
+          if (xt >= XS) {
+            ok = mbar_wait(x_empty + s, (unsigned)(xt / XS - 1) & 1);
+            if (!ok) { atomicExch(err, 56); break; }
+          }
+          mbar_expect_tx(x_full + s, Shape::XSTAGE);
+          f3_tma_3d(smem_u32(xring + s * Shape::XSTAGE), &map_p, c * F3_CHUNK, tile % row_tiles * BN, 0, x_full + s);
+        }
+    }
+  } else if (warp == MMA_WARP) {
+    // The whole warp walks, in uniform registers, and one lane issues: a lane that walks alone moves every operand into them,
+    // 55 cycles an instruction, and each barrier costs it 300.
+    const bool issues = f3_elect();
+    const unsigned base = __shfl_sync(0xffffffffu, tmem, 0);
+    const unsigned long long x0 = tc5_desc(__shfl_sync(0xffffffffu, smem_u32(xring), 0), 16, 1024);
+    constexpr unsigned idesc = f3_idesc(BN);
+    constexpr int wp[6] = {2, 0, 1, 1, 0, 0}, xp[6] = {0, 2, 1, 0, 1, 0};
+    int it = 0, xs = 0;
+    unsigned x_parity = 0;
+    for (int tile = first_tile; tile < tiles && ok; tile += step)
+      for (int c = 0; c < chunks; ++c, ++it) {
+        const int b = it & 1;
+        if ((c & 1) == 0) ok = mbar_wait(x_full + xs, x_parity);
+        if (ok) ok = mbar_wait(ready + b, (unsigned)(it >> 1) & 1);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (issues) atomicExch(err, 57);
+          break;
+        }
+        tc5_fence_after();
+        const bool x_done = (c & 1) || c + 1 == chunks;
+        if (issues) {
+          const unsigned long long xd = x0 + (unsigned)(xs * (Shape::XSTAGE / 16) + (c & 1) * 4);
+#pragma unroll
+          for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int k = 0; k < 2; ++k)          // 16 k: 8 columns of a part of W, 32 bytes along the rows of a part of A
+              tc5_mma_ts(base + b * BN, base + Shape::PARTS + b * 48 + wp[p] * 16 + k * 8, xd + xp[p] * (BN * 128 / 16) + k * 2, idesc, (p | k) != 0);
+          if (x_done) tc5_commit(x_empty + xs);
+          tc5_commit(done + b);
+        }
+        __syncwarp();
+        if (x_done && ++xs == XS) { xs = 0; x_parity ^= 1; }
+      }
+  } else if (warp >= Shape::DRAINS) {
+    // ---- converters ----
+    const int set = (warp - Shape::DRAINS) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+    for (int it = set; it < mine; it += SETS) {
+      const int s = it % WS, b = it & 1;
+      if (ok) {
+        ok = mbar_wait(w_full + s, (unsigned)(it / WS) & 1);
+        if (!ok && lane == 0) atomicExch(err, 58);
+      }
+      const unsigned at = smem_u32(wring + s * Shape::WSTAGE) + row * 128;
+      ulonglong2 v[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = f3_lds(at + ((c ^ (row & 7)) << 4));
+      unsigned p[3][16];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        f3_split(v[c].x, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
+        f3_split(v[c].y, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(w_empty + s);
+      if (it >= 2 && ok) {
+        ok = mbar_wait(done + b, (unsigned)((it >> 1) - 1) & 1);
+        if (!ok && lane == 0) atomicExch(err, 59);
+      }
+      __syncwarp();
+      tc5_fence_after();
+      const unsigned to = tmem + ((unsigned)(quarter * 32) << 16) + Shape::PARTS + b * 48;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) f3_st16(to + q * 16, p[q]);
+      f3_st_wait();
+      tc5_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ready + b);
+    }
+  } else {
+    // ---- drain: this thread's feature, WIDTH rows of the tile ----
+    constexpr int WIDTH = Shape::WIDTH, STEP = Shape::STEP;
+    const int col = (warp >> 2) * WIDTH;
+    const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16) + col;
+    float acc[WIDTH];
+    if (lane < 2) mbar_arrive(ready + lane);                     // both accumulators are free
+    int it = 0;
+    for (int tile = first_tile; tile < tiles; tile += step) {
+      const int m0 = tile % row_tiles * BN + col, n = tile / row_tiles * 128 + (warp & 3) * 32 + lane;
+      for (int c = 0; c < chunks; ++c, ++it) {
+        const int b = it & 1;
+        const bool first = c % F3_BLOCK_CHUNKS == 0, last = c + 1 == chunks;
+        if (ok) {
+          ok = mbar_wait(done + b, (unsigned)(it >> 1) & 1);
+          if (!ok && lane == 0) atomicExch(err, 60);
+        }
+        __syncwarp();
+        tc5_fence_after();
+#pragma unroll
+        for (int j0 = 0; j0 < WIDTH; j0 += STEP) {
+          float v[STEP];
+          f3_ld(lanes + b * BN + j0, v);
+#pragma unroll
+          for (int j = 0; j < STEP; ++j) acc[j0 + j] = first ? v[j] : acc[j0 + j] + v[j];
+        }
+        tc5_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ready + b);
+        if (!last && (c + 1) % F3_BLOCK_CHUNKS != 0) continue;
+        // a block is complete: it joins those before it, or goes to its plane
+        const bool whole = splits == 1;
+#pragma unroll
+        for (int j0 = 0; j0 < WIDTH; j0 += STEP) {
+          float v[STEP];
+          if (whole && c >= F3_BLOCK_CHUNKS) {
+            f3_ld(lanes + Shape::TOTAL + j0, v);
+#pragma unroll
+            for (int j = 0; j < STEP; ++j) acc[j0 + j] = v[j] + acc[j0 + j];
+          }
+          if (whole && !last) {
+#pragma unroll
+            for (int j = 0; j < STEP; ++j) v[j] = acc[j0 + j];
+            f3_st(lanes + Shape::TOTAL + j0, v);
+          }
+        }
+        if ((last || !whole) && n < N) {
+          const float more = whole && bias ? bias[n] : 0.f;
+          const size_t pitch = whole ? ldc : N;
+          float* dst = (whole ? C : planes + (size_t)((c_begin + c) / F3_BLOCK_CHUNKS) * M * N) + m0 * pitch + n;
+          bool finite = true;
+#pragma unroll
+          for (int j = 0; j < WIDTH; ++j, dst += pitch) {
+            finite &= f3_finite(acc[j]);
+            if (m0 + j < M) *dst = acc[j] + more;
+            asm volatile("" : "+l"(dst));        // one address after the other: all of them at once do not fit the registers
+          }
+          if (whole && !finite) f3_again(A, W, C, m0, min(M, m0 + WIDTH), n, K, lda, ldw, ldc, more);
+        }
+        __syncwarp();
+      }
+    }
+  }
+  // every warp gets here (all waits are bounded); then the tensor memory goes back
+  __syncwarp();
+  tc5_fence_before();
+  __syncthreads();
+  if (warp == MMA_WARP) {
+    tc5_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(512) : "memory");
+  }
+}
+
+// The planes of a split product, block by block, + bias; a thread has one element of the output.
+__global__ void __launch_bounds__(256)
+f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+              float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
+  pdl_trigger();
+  pdl_wait();
+  const size_t size = (size_t)M * N;
+  const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK;
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < size; i += (size_t)gridDim.x * 256) {
+    const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
+    float total = 0.f;
+    for (int b0 = 0; b0 < blocks; b0 += 8) {     // eight loads on their way at a time
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __ldcg(planes + (size_t)min(b0 + j, blocks - 1) * size + i);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) total = b0 + j < blocks ? total + v[j] : total;
+    }
+    if (!f3_finite(total)) total = f3_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+    C[(size_t)m * ldc + n] = total + (bias ? bias[n] : 0.f);
+  }
+}
+
+// ---- host -----------------------------------------------------------------------------------------------------------
+// A [rows, K] float matrix of row pitch ld as lines of 32 k: boxes of box_rows x box_lines lines.
+static bool f3_map_lines(CUtensorMap* map, const float* base, int rows, int K, int ld, int box_rows, int box_lines, bool swizzle) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint64_t dims[3] = {32, (cuuint64_t)(K / 32), (cuuint64_t)rows};
+  const cuuint64_t strides[2] = {128, (cuuint64_t)ld * 4};
+  const cuuint32_t box[3] = {32, (cuuint32_t)box_lines, (cuuint32_t)box_rows};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// Boxes of 128 rows x 32 k of W.
+static bool f3_map_w(CUtensorMap* map, const float* base, int rows, int K, int ld) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  const cuuint32_t box[2] = {32, 128};
+  const cuuint32_t estr[2] = {1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// Boxes of the three parts of bn rows x 64 k of A.
+static bool f3_map_parts(CUtensorMap* map, void* base, int M, int K, int bn) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)M, 3};
+  const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)M * K * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)bn, 3};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int MP>
+static int f3_launch_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc,
+                          bool early, int* err, cudaStream_t s) {
+  using Shape = F3Rows<MP>;
+  CUtensorMap mx, mw;
+  if (!f3_map_lines(&mx, A, M, K, lda, MP, F3R_K / 32, false) || !f3_map_lines(&mw, W, N, K, ldw, F3R_FEATURES, 17, true)) return (int)cudaErrorInvalidValue;
+  const cudaError_t e = cudaFuncSetAttribute(f3_rows_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
+  if (e != cudaSuccess) return (int)e;
+  const int sms = device_sm_count(), groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
+  if (sms <= 0) return (int)cudaErrorInvalidDevice;
+  launch(f3_rows_kernel<MP>, dim3(groups < sms ? groups : sms), dim3(Shape::THREADS), Shape::SMEM, s, mx, mw, A, W, bias, C, M, N, K, lda, ldw,
+         ldc, early, err);
+  return launch_status();
+}
+
+int launch_f32x3_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc,
+                     bool early, int* err, cudaStream_t s) {
+  if (M == 1) return f3_launch_rows<1>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
+  if (M == 2) return f3_launch_rows<2>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
+  if (M <= 4) return f3_launch_rows<4>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
+  if (M <= 8) return f3_launch_rows<8>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
+  return f3_launch_rows<16>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
+}
+
+// How f3_tile_kernel takes a product: the width of its tiles, and into how many ranges of blocks a tile is cut.  The one that ends
+// first: the chunks of the fullest SM at what a chunk takes (ns), and for a split the trip through its planes.
+struct F3Plan { int bn, splits; };
+static F3Plan f3_plan(int M, int N, int K, int sms) {
+  const int widths[4] = {128, 96, 64, 32}, ns[4] = {700, 620, 565, 450};
+  const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK;
+  const double planes = 4.0 * blocks * M * N;
+  F3Plan best = {128, 1};
+  double least = -1;
+  for (int i = 0; i < 4; ++i) {
+    const long long tiles = (long long)((M + widths[i] - 1) / widths[i]) * ((N + 127) / 128);
+    const long long room = sms / tiles;
+    const int splits = planes <= 64e6 ? (int)(room < 1 ? 1 : room < blocks ? room : blocks) : 1;
+    double t = splits > 1 ? 8.0 * ((blocks + splits - 1) / splits) * ns[i] + 3000 + planes / 2000 : (double)((tiles + sms - 1) / sms) * (K / F3_CHUNK) * ns[i];
+    if (least < 0 || t < least) { best = {widths[i], splits}; least = t; }
+  }
+  return best;
+}
+static size_t f3_parts_bytes(int M, int K) { return ((size_t)6 * M * K + 255) / 256 * 256; }
+size_t f32x3_scratch(int M, int N, int K) {
+  const int sms = device_sm_count();
+  const F3Plan plan = f3_plan(M, N, K, sms > 0 ? sms : 1);
+  return f3_parts_bytes(M, K) + (plan.splits > 1 ? (size_t)4 * ((K + F3_BLOCK - 1) / F3_BLOCK) * M * N : 0);
+}
+
+template <int BN>
+static int f3_launch_tiles(const float* A, const float* W, const float* bias, float* C, void* parts, float* planes, int splits, int M, int N,
+                           int K, int lda, int ldw, int ldc, bool early, int* err, int sms, cudaStream_t s) {
+  using Shape = F3Tile<BN>;
+  CUtensorMap mp, mw;
+  if (!f3_map_parts(&mp, parts, M, K, BN) || !f3_map_w(&mw, W, N, K, ldw)) return (int)cudaErrorInvalidValue;
+  const cudaError_t e = cudaFuncSetAttribute(f3_tile_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
+  if (e != cudaSuccess) return (int)e;
+  const long long tiles = (long long)((M + BN - 1) / BN) * ((N + 127) / 128);
+  launch(f3_tile_kernel<BN>, dim3((unsigned)(splits > 1 ? tiles * splits : tiles < sms ? tiles : sms)), dim3(Shape::THREADS), Shape::SMEM, s, mp,
+         mw, A, W, bias, C, planes, splits, M, N, K, lda, ldw, ldc, early, err);
+  return launch_status();
+}
+
+int launch_f32x3_many(const float* A, const float* W, const float* bias, float* C, void* scratch, int M, int N, int K, int lda, int ldw, int ldc,
+                      bool early, int* err, cudaStream_t s) {
+  const int sms = device_sm_count();
+  if (sms <= 0) return (int)cudaErrorInvalidDevice;
+  const size_t most = (size_t)sms * 8, eighths = ((size_t)M * (K / 8) + 255) / 256, elements = ((size_t)M * N + 255) / 256;
+  launch(f3_parts_kernel, dim3((unsigned)(eighths < most ? eighths : most)), dim3(256), 0, s, A, (uint4*)scratch, M, K, lda,
+         lda % 4 == 0 && !((uintptr_t)A & 15));
+  const F3Plan plan = f3_plan(M, N, K, sms);
+  float* planes = reinterpret_cast<float*>(static_cast<char*>(scratch) + f3_parts_bytes(M, K));
+  int e;
+  if (plan.bn == 128) e = f3_launch_tiles<128>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  else if (plan.bn == 96) e = f3_launch_tiles<96>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  else if (plan.bn == 64) e = f3_launch_tiles<64>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  else e = f3_launch_tiles<32>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  if (e != 0 || plan.splits == 1) return e;
+  launch(f3_sum_kernel, dim3((unsigned)(elements < most ? elements : most)), dim3(256), 0, s, planes, A, W, bias, C, M, N, K, lda, ldw, ldc);
+  return launch_status();
+}

@@ -38,7 +38,7 @@ NVCC_FLAGS = [
 # "delta" the gated delta rule.  A library is compiled when a model first asks for one of its kernels, so a run compiles only what
 # its model and dtype need.
 LIBRARIES: Dict[str, List[str]] = {
-    "core": ["elementwise.cu", "rope_cache.cu", "attention_generic.cu", "attention_f32.cu", "gemm_f32.cu", "sampling.cu", "step.cu"],
+    "core": ["elementwise.cu", "rope_cache.cu", "attention_generic.cu", "attention_f32.cu", "gemm_f32.cu", "gemm_f32x3.cu", "sampling.cu", "step.cu"],
     "chain": ["gemm_chain.cu"],
     "tcgen05": ["gemm_tcgen05.cu"],
     "bf16": ["attention_mma.cu", "attention_tcgen05.cu"],

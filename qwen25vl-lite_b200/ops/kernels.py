@@ -64,7 +64,7 @@ _SIGNATURES = {
 _UNTYPED = {
     "q25_attention_decode_bf16": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "q25_attention_prefill_bf16": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _P],
-    "q25_gemm_f32": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "q25_gemm_f32": [_P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "q25_gemm_tcgen05_bf16": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _P],
     "q25_paged_attention_f32": [_P, _I, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P, _P],
     "q25_sample_rows": [_P, _LL, _I, _I, _P, _P, _P, _P, _P, _P],
@@ -478,6 +478,9 @@ def attention_prefill_tcgen05(qkv: torch.Tensor, out: torch.Tensor, k_pages: tor
         count_replayed(1)                      # the merge kernel, launched by the same call
 
 
+F32X3_FEW = 16                # rows that the 32-bit product on tensor cores takes as they are (csrc/gemm_f32x3.cuh)
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, fixed: bool = False) -> None:
     """out[M,N] = a[M,K] . w[N,K]^T + bias, plain float32 FMA.  ``fixed``: ``w`` is a weight that no kernel writes, and is fetched
     before the kernel ahead on the stream has ended."""
@@ -488,8 +491,14 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     for t, what in ((a, "a"), (w, "w"), (out, "out")):
         if t.dtype != torch.float32 or not t.is_cuda or t.stride(1) != 1:
             raise KernelError(f"gemm_f32 {what}: needs a float32 CUDA matrix with unit inner stride")
+    lda = a.stride(0) if m > 1 else k
+    scratch = None            # the three bfloat16 parts of a's values, and sums of parts of K, where the tensor cores take more than a few rows
+    if k >= 256 and k % 32 == 0 and (m > F32X3_FEW or lda % 4 or lda < k or a.data_ptr() % 16):
+        size = _fn("q25_gemm_f32_scratch", [_I, _I, _I])
+        size.restype = _LL
+        scratch = torch.empty(size(m, n, k), dtype=torch.uint8, device=a.device)
     _check(_fn("q25_gemm_f32", _UNTYPED["q25_gemm_f32"])(
-        a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), m, n, k, a.stride(0), w.stride(0), out.stride(0),
+        a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _ptr(scratch), m, n, k, lda, w.stride(0), out.stride(0),
         int(fixed), error_flag(out.device).data_ptr(), _stream()), "gemm_f32")
 
 

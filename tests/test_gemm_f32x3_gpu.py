@@ -1,0 +1,60 @@
+"""The 32-bit product on tensor cores: every kernel gives a row the same bits, no further from 64 bits than 32-bit additions put it, at the
+edges of its tiles; operands that have no three bfloat16 parts come out as plain FMA has them."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _product(a, w, b=None):
+    from qwen25vl_lite.ops import kernels
+    out = torch.full((a.shape[0], w.shape[0]), float("nan"), device="cuda")
+    kernels.gemm_f32(a, w, b, out, fixed=True)
+    assert int(kernels.error_flag(out.device)) == 0
+    return out
+
+
+#  rows, features, K, pitch of the rows beyond K: up to 16 rows a stream; more of them tiles of 32, 64, 96 and 128 rows, with K in parts (where the
+#  tiles are few) and whole
+CASES = [(1, 15, 256, 0), (2, 33, 288, 0), (3, 3000, 512, 4), (8, 2048, 544, 0), (9, 100, 1056, 0), (16, 16, 11008, 32),
+         (17, 127, 256, 0), (33, 129, 288, 0), (64, 2048, 2048, 0), (65, 7000, 320, 4), (97, 9472, 512, 0), (200, 9500, 800, 0), (300, 20000, 256, 12), (1000, 640, 4096, 0)]
+
+
+@pytest.mark.parametrize("m,n,k,extra", CASES)
+def test_rows_have_the_same_bits_in_every_kernel(m, n, k, extra):
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a = torch.randn(m, k + extra, generator=gen, device="cuda")[:, :k]
+    w, b = torch.randn(n, k, generator=gen, device="cuda"), torch.randn(n, generator=gen, device="cuda")
+    out = _product(a, w, b)
+    # parts: 2^-24 of the operands' product is left out.  A chunk of 32 k has 12 tensor-core additions, each cut off at 2^-23 of
+    # at most the sum of the magnitudes; its value meets up to 7 others in its block, which meets the blocks before, then the bias.
+    want, size = a.double() @ w.double().T + b.double(), a.double().abs() @ w.double().abs().T + b.double().abs()
+    assert ((out.double() - want).abs() <= (1 + 2 * 12 + 8 + -(-k // 256) + 1) * 2.0 ** -24 * size).all()
+    for rows in (1, 2, 4, 7, 16, 17, 50, 130):
+        if rows < m:
+            assert torch.equal(_product(a[m - rows:], w, b), out[m - rows:]), rows
+
+
+@pytest.mark.parametrize("m", [5, 60])
+def test_rows_that_are_not_aligned(m):
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    flat, w = torch.randn(m * 513 + 3, generator=gen, device="cuda"), torch.randn(300, 512, generator=gen, device="cuda")
+    for first, pitch in ((1, 512), (0, 513)):
+        a = flat[first:].as_strided((m, 512), (pitch, 1))
+        assert torch.equal(_product(a, w), _product(a.clone(), w))
+
+
+@pytest.mark.parametrize("m,n", [(3, 260), (16, 260), (40, 260), (300, 260), (300, 9600)])
+def test_operands_without_three_parts(m, n):
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, w = torch.randn(m, 512, generator=gen, device="cuda"), torch.randn(n, 512, generator=gen, device="cuda")
+    a[1, 0] = 0.5
+    clean = _product(a, w)
+    a[m - 1, 7], a[0, 500], w[3, 40], w[259, 0] = float("inf"), float("nan"), float("-inf"), 3.4e38    # the last rounds up to infinity in 16 bits
+    want = a.double() @ w.double().T
+    want[want.abs() > 3.4028235e38] = want[want.abs() > 3.4028235e38].sign() * float("inf")
+    out = _product(a, w)
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isposinf(), want.isposinf()) and torch.equal(out.isneginf(), want.isneginf())
+    assert torch.equal(out[1:m - 1, 4:259], clean[1:m - 1, 4:259])
+    assert abs(float(out[1, 259]) / float(want[1, 259]) - 1) < 1e-6
