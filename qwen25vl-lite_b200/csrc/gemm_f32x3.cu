@@ -100,9 +100,13 @@ __device__ __forceinline__ void f3_tma_3d_once(unsigned dst, const CUtensorMap* 
 // seen as lines of 32; a row of W's box holds 17 of them, the last one not used, so that the 128-byte swizzle puts the same
 // line of eight rows into eight different bank groups.  Four warps share a stage, half a block each: the weights are
 // the 16-row side of mma.sync m16n8k16, the rows of x its 8 columns (two such tiles for 9 to 16 rows), and a thread's 16 bytes
-// of a row fill its four k slots (the sum over 16 k has no order).  A chunk's 12 MMAs wait for one another, so it takes many
-// warps to keep up with the copies.  The warp of a block's second half adds its chunks to the first half's sum, in shared
-// memory, where one more warp adds the blocks.
+// of a row fill its four k slots (the sum over 16 k has no order).  A chunk takes some 700 cycles, its 12 MMAs waiting for one
+// another, so it takes many warps to keep up with the copies.  The warp of a block's second half adds its chunks to the first
+// half's sum, in shared memory, where one more warp adds the blocks.
+// Measured, us for 1 / 8 / 16 rows: 151,936 features x 2,048 180 / 195 / 265 (6.9 TB/s; by FMA 176 / 230 / 440), 22,016 x 2,048
+// 32 / 35 / 47 (27 / 40 / 71), 2,048 x 11,008 19 / 20 / 28 (16 / 25 / 41): the end of a product, when the last stages' chunks are
+// on their way, is longer than by FMA.  Two warps a stage: 35, 21; stages of 256 k: 39, 23; sixteen warps with a chunk each of every
+// stage, which is free at once: 37, 22 (every warp pays for every stage's barriers).
 #define F3R_FEATURES 16
 #define F3R_K 512
 #define F3R_PITCH (17 * 128)                     // bytes between the rows of W in a stage
@@ -232,8 +236,9 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const unsigned wa = smem_u32(smem + s * Shape::STAGE) + f * F3R_PITCH + line0;
   const unsigned xa = smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES + (g & (MP < 8 ? MP - 1 : 7)) * (F3R_K * 4) + line0 + t * 16;
   float* slot = red + s * Shape::RED + block * (F3R_FEATURES * MP) + f;
+  // Past the end of K the copies bring zeros, which are multiplied like the rest: a branch around a chunk would keep the compiler from
+  // working on two at a time (22,016 features x 2,048, one row: 32.5 -> 31.8 us; 2,048 x 11,008: 25.3 -> 19.2).
   for (int i = s; i < items; i += S, parity ^= 1) {
-    const int left = (K - i % spans * F3R_K - block * F3_BLOCK) / F3_CHUNK - half * 4;        // chunks; may be <= 0
     float v[4][TILES][4];
     if (ok) {
       ok = mbar_wait(full + s, parity);
@@ -243,7 +248,6 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     for (int c = 0; c < 4; ++c) {
 #pragma unroll
       for (int n = 0; n < TILES; ++n) v[c][n][0] = v[c][n][1] = v[c][n][2] = v[c][n][3] = 0.f;
-      if (c >= left) continue;
       unsigned a[2][3][4], b[TILES][2][3][2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
