@@ -32,6 +32,7 @@ from ..cache.manager import CacheManager, RequestCache
 from ..models.decoder import DecoderModel, StopRuntime
 from ..ops import kernels
 from ..ops.attention import Workspace
+from ..ops.host import host_ints
 
 
 @dataclass(eq=False)
@@ -207,6 +208,7 @@ class ModelRunner:
         self._staging_free, self._step_done = (torch.cuda.Event(), torch.cuda.Event()) if self.device.type == "cuda" else (None, None)
         self._stream = (None, None)             # the stream of the last step: its handle, and torch's object for it
         self._reserve(max_step_tokens * (3 + self.axes + len(self.cache.groups)) + 4096)
+        self._counting = np.arange(256, dtype=np.int32)
         self.live: Dict[object, Request] = {}
         self.steps = 0
         # Steps that bring one token per request are launch-bound (hundreds of small kernels), so
@@ -228,6 +230,7 @@ class ModelRunner:
         # kernels with bounded waits report a wait that gave up here; written behind every step's kernels
         # and looked at before the next one
         self._error_host = torch.zeros(1, dtype=torch.int32, pin_memory=self.device.type == "cuda")
+        self._error_np = self._error_host.numpy()
 
     def __del__(self):
         if getattr(self, "_step_done", None) is not None and _let_go is not None:
@@ -258,6 +261,12 @@ class ModelRunner:
         self._staging = torch.empty(n_ints, dtype=torch.int32, pin_memory=pin)
         self._staging_np = self._staging.numpy()
         self._device_ints = torch.empty(n_ints, dtype=torch.int32, device=self.device)
+
+    def _count_to(self, n: int) -> np.ndarray:
+        """0 .. n - 1 (not to be written to)."""
+        if self._counting.shape[0] < n:
+            self._counting = np.arange(max(n, 256), dtype=np.int32)
+        return self._counting[:n]
 
     def _record(self, event) -> None:
         """``event.record()`` without building the current stream's object anew (4 us, twice a step)."""
@@ -415,15 +424,15 @@ class ModelRunner:
 
         # ---- pack ----
         host = HostStep(q_lens, starts, N, S)
-        plans = {key: {name: np.ascontiguousarray(a, dtype=np.int32).reshape(-1)
-                       for name, a in part.plan_step(host).items()} for key, part in self._planners.items()}
+        flat = lambda a: a if a.dtype == np.int32 and a.ndim == 1 else np.ascontiguousarray(a, dtype=np.int32).reshape(-1)
+        plans = {key: {name: flat(np.asarray(a)) for name, a in part.plan_step(host).items()} for key, part in self._planners.items()}
         n_work = sum(a.shape[0] + 4 for p in plans.values() for a in p.values())
         total = (N * (2 + self.axes + len(groups)) + (S + 1) + 2 * S + M + S * sum(widths) + n_work
                  + 4 * (8 + 2 * len(groups)))
         self._reserve(total)
         if self._staging_free is not None:
             self._staging_free.synchronize()               # the last copy out of the staging buffer is done
-        buf = self._staging_np
+        buf, at = self._staging_np, self._staging.data_ptr()
         off = 0
 
         def take(n):
@@ -453,45 +462,51 @@ class ModelRunner:
                 view, plan_s[key, name] = take(a.shape[0])
                 view[:] = a
 
+        def fill(span, numbers):
+            if not host_ints(numbers, span[1], at + 4 * span[0]):
+                buf[span[0]:span[0] + span[1]] = numbers
+
         cu[0] = 0
-        last_position = []
+        last_position, highest = [], None
         if (max(q_lens) == 1 and all(e.positions is None for e in entries)
                 and getattr(self.position, "default_is_linear", False)):
             # A step of single tokens at their default positions (the usual decode step): the
             # arrays are filled for all entries at once, and a request's block table is converted
             # only when it has grown.
-            ids = np.fromiter((e.tokens[0] for e in entries), dtype=np.int64, count=real)
-            if ids.min() < 0 or ids.max() >= self.vocab_size:
+            # Lists of a few numbers are cheaper than numpy's arrays of them.
+            caches = [e.request.cache for e in entries]
+            ids = [int(e.tokens[0]) for e in entries]
+            if min(ids) < 0 or max(ids) >= self.vocab_size:
                 raise ValueError(f"token id outside [0, {self.vocab_size}) in a decode step")
-            st = np.asarray(starts, dtype=np.int64)
-            place = st.copy()
-            place[:real] += np.fromiter((e.request.cache.position_offset for e in entries), dtype=np.int64, count=real)
-            tok[:real] = ids
-            tok[real:] = 0
-            pos[:, :] = place
-            last_position = place[:real].tolist()
-            tseq[:] = np.arange(S)
-            cu[1:] = np.arange(1, S + 1)
-            qs[:] = st
-            sl[:real] = [e.request.cache.slot for e in entries]
-            r = 0
-            for i, e in enumerate(entries):
-                for w_ in e.want:
-                    if int(w_) != 0:
-                        raise ValueError(f"wanted place {w_} is outside the 1 token of the entry")
-                    rows[r] = i
-                    r += 1
-            if pad:
-                sl[real:] = pad_cache.slot
-                rows[real:] = np.arange(real, S)
-            for g, gs, gt in zip(groups, g_slot, g_tab):
-                for i, (e, s0) in enumerate(zip(entries, starts)):
+            last_position = [s0 + c.position_offset for c, s0 in zip(caches, starts)]
+            highest = max(last_position)
+            zeros = [0] * pad
+            count = self._count_to(S + 1)
+            fill(tok_s, ids + zeros)
+            for a in range(self.axes):
+                fill((pos_s[0] + a * N, N), last_position + zeros)
+            tseq[:] = count[:S]
+            cu[:] = count
+            fill(qs_s, starts)
+            fill(sl_s, [c.slot for c in caches] + ([pad_cache.slot] * pad if pad else []))
+            if graph_key is not None:                      # every entry wants its one place
+                rows[:] = count[:M]
+            else:
+                r = 0
+                for i, e in enumerate(entries):
+                    for w_ in e.want:
+                        if int(w_) != 0:
+                            raise ValueError(f"wanted place {w_} is outside the 1 token of the entry")
+                        rows[r] = i
+                        r += 1
+            for g, gs_s, gt in zip(groups, g_slot_s, g_tab):
+                fill(gs_s, [c.tables[g.index][s0 // ps] * ps + s0 % ps for c, s0 in zip(caches, starts)]
+                     + ([pad_cache.tables[g.index][0] * ps] * pad if pad else []))
+                for i, e in enumerate(entries):
                     table = e.request.block_table(g.index)
-                    gs[i] = e.request.cache.tables[g.index][s0 // ps] * ps + s0 % ps
                     gt[i, :len(table)] = table
                     gt[i, len(table):] = 0
                 if pad:
-                    gs[real:] = pad_cache.tables[g.index][0] * ps
                     gt[real:, :] = 0
                     gt[real:, 0] = pad_cache.tables[g.index][0]
         else:
@@ -560,7 +575,7 @@ class ModelRunner:
                     gt[i, len(table):] = 0
 
         limit = getattr(self.position, "limit", None)
-        if limit is not None and N and int(pos.max()) >= limit:
+        if limit is not None and N and (int(pos.max()) if highest is None else highest) >= limit:
             raise ValueError(f"a token sits at position {int(pos.max())}, the model places positions 0 to {limit - 1}")
         return lambda tokens=None, device_ids=None: self._run_packed(
             tokens, entries, q_lens, starts, widths, graph_key, off, N, S, M, ps, tok, tok_s, pos_s, tseq_s, cu_s, qs_s, sl_s,
@@ -658,7 +673,7 @@ class ModelRunner:
         bounded waits (the flag travels to the host after every step, behind the step's kernels
         and before anything that reads its logits).  The flag is cleared, so that one failed
         step does not condemn the steps after it."""
-        code = int(self._error_host[0])
+        code = int(self._error_np[0])
         if code != 0:
             self._error_host.zero_()
             if self.device.type == "cuda":

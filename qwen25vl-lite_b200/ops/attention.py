@@ -41,11 +41,12 @@ _plans: "OrderedDict[tuple, Dict[str, np.ndarray]]" = OrderedDict()
 PLANS_KEPT = 16
 
 
-def _remembered(kind: str, args: tuple, host, build) -> Dict[str, np.ndarray]:
+def _remembered(kind: str, args: tuple, host, build, starts: bool = True) -> Dict[str, np.ndarray]:
     """The work lists of a step's shape, built once: mixers of one model that differ in what their plans hold ask for
     the same lists within a step, and prompts cut into portions of one size bring the same shape step after step.
+    ``starts`` False: the lists do not depend on where the entries' tokens stand.
     The arrays are shared and not to be written to; the dictionary is the caller's."""
-    key = (kind, args, tuple(host.q_lens), tuple(host.starts))
+    key = (kind, args, tuple(host.q_lens), tuple(host.starts) if starts else None)
     lists = _plans.get(key)
     if lists is None:
         lists = _plans[key] = build()
@@ -69,6 +70,8 @@ def plan_step(host, group: int, window: int = 0, places: int = 0) -> Dict[str, n
     ``merge128``: the tiles whose parts a second kernel adds up, as (entry, tile, first part, parts);
     ``pairs128`` is not empty when ``tiles128`` is meant for clusters of two CTAs (``pair_split``).
     ``places``: CTAs of the tcgen05 kernel that run at a time for one kv head (0: nothing is cut)."""
+    if group <= 16 and max(host.q_lens) == 1:     # no runs: the same lists wherever the tokens stand
+        return _remembered("rows", (group, window, places), host, lambda: _plan_step(host, group, window, places), starts=False)
     return _remembered("rows", (group, window, places), host, lambda: _plan_step(host, group, window, places))
 
 

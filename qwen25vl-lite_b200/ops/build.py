@@ -35,7 +35,7 @@ NVCC_FLAGS = [
 # rotation of part of a head in either pairing, "latent" the compressed cache row of latent attention,
 # "retention" the decayed linear attention, "memory" the matrix memories whose gates depend on the token, "hyper" a
 # residual stream of several rows per token, "state_space" the tensor-core runs of the state space, "differential" attention whose heads subtract one map from another,
-# "delta" the gated delta rule.  A library is compiled when a model first asks for one of its kernels, so a run compiles only what
+# "delta" the gated delta rule, "host" what the host does with Python's lists.  A library is compiled when a model first asks for one of its kernels, so a run compiles only what
 # its model and dtype need.
 LIBRARIES: Dict[str, List[str]] = {
     "core": ["elementwise.cu", "rope_cache.cu", "attention_generic.cu", "attention_f32.cu", "gemm_f32.cu", "gemm_f32x3.cu", "sampling.cu", "step.cu"],
@@ -53,6 +53,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "state_space": ["state_space.cu"],
     "differential": ["attention_differential.cu"],
     "delta": ["delta_rule.cu"],
+    "host": ["host.cpp"],
 }
 
 

@@ -24,6 +24,7 @@ import numpy as np
 import torch
 
 from ..ops import kernels
+from ..ops.host import host_ints
 from .params import SamplingParams
 
 
@@ -141,28 +142,25 @@ class Sampler:
         if len(params) < rows:
             raise ValueError(f"{rows} rows of logits and what {len(params)} of them ask for")
         params = params[:rows]
-        lists = array("i")
-        spans = []
+        spans, lists, n = [], [], 0
         for p, prev in zip(params, previous or [()] * rows):
-            begin = len(lists)
+            begin = n
             if p.has_penalties and prev:
-                try:
-                    lists.extend(prev)
-                except TypeError:                      # numbers that are no ints, or an array of other ints
-                    del lists[begin:]
-                    lists.extend(int(t) for t in prev)
-            spans.append((begin, len(lists)))
-        spans += [(len(lists), len(lists))] * (rows - len(spans))
+                if type(prev) is not list:
+                    prev = self._ints(prev)
+                n += len(prev)
+                lists.append((begin, n, prev))
+            spans.append((begin, n))
+        spans += [(n, n)] * (rows - len(spans))
         words = rows * kernels.SAMPLE_ASK_WORDS
-        staged = torch.empty(words + max(len(lists), 1), dtype=torch.int32, pin_memory=True)
+        staged = torch.empty(words + max(n, 1), dtype=torch.int32, pin_memory=True)
         host = staged.numpy()
         asks = host[:words].reshape(rows, kernels.SAMPLE_ASK_WORDS)
         floats = asks.view(np.float32)
-        filters = [p.has_filters for p in params]
-        asks[:, 1] = [max(0, min(int(p.top_k or 0), 1 << 30)) if f else 0 for p, f in zip(params, filters)]
-        floats[:, 0] = [p.temperature for p in params]
-        floats[:, 2] = [p.min_p if f else 0.0 for p, f in zip(params, filters)]
-        floats[:, 3] = [p.top_p if f else 1.0 for p, f in zip(params, filters)]
+        floats[:, (0, 2, 3, 7, 8, 9)] = [
+            (p.temperature, p.min_p, p.top_p, p.repetition_penalty, p.presence_penalty, p.frequency_penalty) if p.has_filters else
+            (p.temperature, 0.0, 1.0, p.repetition_penalty, p.presence_penalty, p.frequency_penalty) for p in params]
+        asks[:, 1] = [max(0, min(int(p.top_k or 0), 1 << 30)) if p.has_filters else 0 for p in params]
         if any(p.temperature > 0 for p in params):
             seed = np.array([int(s) & ((1 << 64) - 1) for s in list(seeds)[:rows]], dtype=np.uint64)
             asks[:, 4] = seed.astype(np.uint32).view(np.int32)
@@ -170,12 +168,22 @@ class Sampler:
             asks[:, 6] = [int(t) for t in list(token_indices)[:rows]]
         else:
             asks[:, 4:7] = 0
-        floats[:, 7] = [p.repetition_penalty for p in params]
-        floats[:, 8] = [p.presence_penalty for p in params]
-        floats[:, 9] = [p.frequency_penalty for p in params]
         asks[:, 10:12] = spans
-        host[words:words + len(lists)] = np.frombuffer(lists, dtype=np.int32) if lists else 0
+        if n == 0:
+            host[words] = 0
+        for begin, end, prev in lists:
+            if type(prev) is not list or not host_ints(prev, end - begin, staged.data_ptr() + 4 * (words + begin)):
+                host[words + begin:words + end] = np.frombuffer(self._ints(prev), dtype=np.int32)
         return staged.to(self.device, non_blocking=True)
+
+    @staticmethod
+    def _ints(numbers) -> array:
+        out = array("i")
+        try:
+            out.extend(numbers)
+        except TypeError:                      # numbers that are no ints, or an array of other ints
+            out = array("i", [int(t) for t in numbers])
+        return out
 
     def _copy_back(self, out: torch.Tensor, rows: int):
         if self.device.type != "cuda":
