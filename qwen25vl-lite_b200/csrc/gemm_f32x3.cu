@@ -344,6 +344,10 @@ f3_parts_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, i
 // Warps: 4 drain a tile of up to 64 rows, 8 a wider one (half of its columns each, which is what their registers hold); then 4
 // converters, or 8 where a chunk's MMAs leave less time (the second four take the odd chunks); a producer for W, which runs ahead
 // of the kernel before, one for A's parts, and the MMA warp.
+// Measured, 1,500 rows x 22,016 x 2,048: 586 us, 231 TFLOP/s of the product asked for (by FMA 2,988 us); a chunk takes 654 / 551 / 455 /
+// 420 ns with tiles of 128 / 96 / 64 / 32 rows, which is the same 61 bytes a ns from L2 into every SM (9 TB/s) for all four: the tensor
+// pipe is busy 410 of the 654.  What the warps do between their barriers must stay short: with selects for a block's first chunk
+// (and the spills they brought), an error path in each loop and branches around the arrivals it was 814 ns.
 template <int BN> struct F3Tile {
   static constexpr int XSTAGE = 3 * BN * 128, WSTAGE = 128 * 128;
   static constexpr int XS = BN >= 96 ? 3 : 4;
@@ -384,6 +388,9 @@ __device__ __forceinline__ void f3_st(unsigned taddr, const float (&v)[16]) {
   for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(v[i]);
   f3_st16(taddr, r);
   f3_st_wait();
+}
+__device__ __forceinline__ void f3_arrive(unsigned long long* bar, int lane) {       // by the first lane, without a branch
+  asm volatile("{\n .reg .pred p;\n setp.eq.s32 p, %1, 0;\n @p mbarrier.arrive.shared::cta.b64 _, [%0];\n}\n" ::"r"(smem_u32(bar)), "r"(lane) : "memory");
 }
 __device__ __forceinline__ bool f3_elect() {
   unsigned e;
@@ -513,10 +520,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
     const int set = (warp - Shape::DRAINS) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
     for (int it = set; it < mine; it += SETS) {
       const int s = it % WS, b = it & 1;
-      if (ok) {
-        ok = mbar_wait(w_full + s, (unsigned)(it / WS) & 1);
-        if (!ok && lane == 0) atomicExch(err, 58);
-      }
+      ok = ok && mbar_wait(w_full + s, (unsigned)(it / WS) & 1);
       const unsigned at = smem_u32(wring + s * Shape::WSTAGE) + row * 128;
       ulonglong2 v[8];
 #pragma unroll
@@ -528,12 +532,8 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
         f3_split(v[c].y, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(w_empty + s);
-      if (it >= 2 && ok) {
-        ok = mbar_wait(done + b, (unsigned)((it >> 1) - 1) & 1);
-        if (!ok && lane == 0) atomicExch(err, 59);
-      }
-      __syncwarp();
+      f3_arrive(w_empty + s, lane);
+      if (it >= 2) ok = ok && mbar_wait(done + b, (unsigned)((it >> 1) - 1) & 1);
       tc5_fence_after();
       const unsigned to = tmem + ((unsigned)(quarter * 32) << 16) + Shape::PARTS + b * 48;
 #pragma unroll
@@ -541,37 +541,35 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
       f3_st_wait();
       tc5_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ready + b);
+      f3_arrive(ready + b, lane);
     }
   } else {
     // ---- drain: this thread's feature, WIDTH rows of the tile ----
     constexpr int WIDTH = Shape::WIDTH, STEP = Shape::STEP;
     const int col = (warp >> 2) * WIDTH;
     const unsigned lanes = tmem + ((unsigned)((warp & 3) * 32) << 16) + col;
-    float acc[WIDTH];
+    float acc[WIDTH];                                            // a block's chunks so far
+#pragma unroll
+    for (int j = 0; j < WIDTH; ++j) acc[j] = 0.f;
     if (lane < 2) mbar_arrive(ready + lane);                     // both accumulators are free
     int it = 0;
     for (int tile = first_tile; tile < tiles; tile += step) {
       const int m0 = tile % row_tiles * BN + col, n = tile / row_tiles * 128 + (warp & 3) * 32 + lane;
       for (int c = 0; c < chunks; ++c, ++it) {
         const int b = it & 1;
-        const bool first = c % F3_BLOCK_CHUNKS == 0, last = c + 1 == chunks;
-        if (ok) {
-          ok = mbar_wait(done + b, (unsigned)(it >> 1) & 1);
-          if (!ok && lane == 0) atomicExch(err, 60);
-        }
-        __syncwarp();
+        const bool last = c + 1 == chunks;
+        ok = ok && mbar_wait(done + b, (unsigned)(it >> 1) & 1);
         tc5_fence_after();
 #pragma unroll
         for (int j0 = 0; j0 < WIDTH; j0 += STEP) {
           float v[STEP];
           f3_ld(lanes + b * BN + j0, v);
 #pragma unroll
-          for (int j = 0; j < STEP; ++j) acc[j0 + j] = first ? v[j] : acc[j0 + j] + v[j];
+          for (int j = 0; j < STEP; ++j) acc[j0 + j] += v[j];
         }
         tc5_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(ready + b);
+        f3_arrive(ready + b, lane);
         if (!last && (c + 1) % F3_BLOCK_CHUNKS != 0) continue;
         // a block is complete: it joins those before it, or goes to its plane
         const bool whole = splits == 1;
@@ -603,10 +601,13 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
           if (whole && !finite) f3_again(A, W, C, m0, min(M, m0 + WIDTH), n, K, lda, ldw, ldc, more);
         }
         __syncwarp();
+#pragma unroll
+        for (int j = 0; j < WIDTH; ++j) acc[j] = 0.f;
       }
     }
   }
   // every warp gets here (all waits are bounded); then the tensor memory goes back
+  if (!ok && lane == 0) atomicExch(err, 58);
   __syncwarp();
   tc5_fence_before();
   __syncthreads();
@@ -703,7 +704,7 @@ int launch_f32x3_few(const float* A, const float* W, const float* bias, float* C
 // first: the chunks of the fullest SM at what a chunk takes (ns), and for a split the trip through its planes.
 struct F3Plan { int bn, splits; };
 static F3Plan f3_plan(int M, int N, int K, int sms) {
-  const int widths[4] = {128, 96, 64, 32}, ns[4] = {700, 620, 565, 450};
+  const int widths[4] = {128, 96, 64, 32}, ns[4] = {640, 540, 455, 425};
   const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK;
   const double planes = 4.0 * blocks * M * N;
   F3Plan best = {128, 1};
