@@ -1,8 +1,10 @@
-// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) in true 32-bit: plain FMA on the CUDA cores, no tensor
-// cores and no reduced-precision matrix mode.  This is the matrix product of the 32-bit path
-// (the reference's tested path is float32 end to end, src/qwen25vl_lite/engine.py:63).
+// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) in true 32-bit.  This is the matrix product of the 32-bit path
+// (the reference's tested path is float32 end to end, src/qwen25vl_lite/engine.py:63).  Where K is 256 or more and a multiple of
+// 32 it runs on tensor cores, every number in three exact parts (gemm_f32x3.cu); this file has the others, plain FMA on the
+// CUDA cores.  (Figures below of longer K are from when these kernels took it.  The line lies at 256 because a row of 320 features
+// takes 2.0 us here and 3.3 there, where the start of a product counts for more; from 17 rows on 5.4 and 7.1.)
 //
-// Every output element is summed in one order, which all kernels here share: K is cut into
+// Every output element is summed in one order, which all kernels of this file share: K is cut into
 // segments of 128; inside a segment the even and the odd k are one chain of fma each, in order,
 // and the segment's value is even + odd; the segments' values are added in order; then + bias.
 // The order depends on nothing but K, so a token's result is bit-identical whether it is computed

@@ -479,11 +479,13 @@ def attention_prefill_tcgen05(qkv: torch.Tensor, out: torch.Tensor, k_pages: tor
 
 
 F32X3_FEW = 16                # rows that the 32-bit product on tensor cores takes as they are (csrc/gemm_f32x3.cuh)
+F32X3_SCRATCH = 1 << 28       # bytes that the parts of a product's rows may take; more rows go in several launches (the bits are the same)
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, fixed: bool = False) -> None:
-    """out[M,N] = a[M,K] . w[N,K]^T + bias, plain float32 FMA.  ``fixed``: ``w`` is a weight that no kernel writes, and is fetched
-    before the kernel ahead on the stream has ended."""
+    """out[M,N] = a[M,K] . w[N,K]^T + bias in true 32 bits: by FMA, or from K 256 on (multiples of 32) on tensor cores with every number
+    cut into three exact parts.  A row's bits depend on nothing but K.  ``fixed``: ``w`` is a weight that no kernel writes, and is
+    fetched before the kernel ahead on the stream has ended."""
     m, k = a.shape
     n = w.shape[0]
     if w.shape[1] != k or out.shape[0] != m or out.shape[1] != n:
@@ -494,6 +496,11 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     lda = a.stride(0) if m > 1 else k
     scratch = None            # the three bfloat16 parts of a's values, and sums of parts of K, where the tensor cores take more than a few rows
     if k >= 256 and k % 32 == 0 and (m > F32X3_FEW or lda % 4 or lda < k or a.data_ptr() % 16):
+        slab = max(384, F32X3_SCRATCH // (6 * k) // 384 * 384)              # whole tiles of 128 and of 96 rows
+        if m > slab:
+            for at in range(0, m, slab):
+                gemm_f32(a[at:at + slab], w, bias, out[at:at + slab], fixed)
+            return
         size = _fn("q25_gemm_f32_scratch", [_I, _I, _I])
         size.restype = _LL
         scratch = torch.empty(size(m, n, k), dtype=torch.uint8, device=a.device)

@@ -1,7 +1,8 @@
 """Matrix products of the forward pass: ``y = x . W^T (+ b)``.
 
-* float32: the engine's own FMA kernel (``csrc/gemm_f32.cu``), whose per-element summation
-  order is fixed, so results do not depend on the batch.  No library, no TF32.
+* float32: the engine's own kernels, every number in three exact bfloat16 parts on tensor cores (``csrc/gemm_f32x3.cu``)
+  or, where K is short, FMA (``csrc/gemm_f32.cu``).  The per-element summation order is fixed, so results do not depend
+  on the batch.  No library, no TF32.
 * bfloat16, at most 8 rows (decode steps): the engine's weight-streaming kernel
   (``csrc/gemm_chain.cu``).  It can normalise its input on the fly (a ``DeferredNorm``)
   and add its result into the float32 residual stream, which removes the norm kernels and

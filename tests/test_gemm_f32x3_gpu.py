@@ -58,3 +58,12 @@ def test_operands_without_three_parts(m, n):
     assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isposinf(), want.isposinf()) and torch.equal(out.isneginf(), want.isneginf())
     assert torch.equal(out[1:m - 1, 4:259], clean[1:m - 1, 4:259])
     assert abs(float(out[1, 259]) / float(want[1, 259]) - 1) < 1e-6
+
+
+def test_rows_beyond_the_scratch_limit(monkeypatch):
+    from qwen25vl_lite.ops import kernels
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    a, w, b = (torch.randn(*shape, generator=gen, device="cuda") for shape in ((1000, 256), (300, 256), (300,)))
+    whole = _product(a, w, b)
+    monkeypatch.setattr(kernels, "F32X3_SCRATCH", 1)
+    assert torch.equal(_product(a, w, b), whole)
