@@ -1,7 +1,8 @@
 // C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) of 32-bit operands on the tensor cores, no less precise than by 32-bit FMAs.
 //
 // A 32-bit number is the sum of three bfloat16 numbers, hi + mid + lo: hi is the number rounded, mid what hi leaves, rounded,
-// lo the rest; 8 bits of the mantissa each, so nothing is lost.  Of the nine products of two such sums the six largest are taken;
+// lo the rest; 8 bits of the mantissa each, so nothing is lost (below 2^-109 the rest is less than bfloat16's smallest number, and low
+// bits are lost: of a sum in which such operands alone count, 2e-6 at 2^-116).  Of the nine products of two such sums the six largest are taken;
 // the others (mid lo, lo mid, lo lo) are below 2^-24 of the product.  bfloat16 products are exact in 32 bits, what remains is how
 // they are added.  The tensor core cuts bits off where FMA rounds, so it adds no more than 32 k (two instructions of 16 k for
 // each of the six, the small ones first); the values of these chunks are added by ordinary 32-bit additions.  For every
@@ -14,6 +15,9 @@
 //
 // The order depends on nothing but K, so a token's result is bit for bit the same whether it is computed alone, in a portion or in a
 // large batch: mma.sync and tcgen05.mma give the same bits for the same 16 k (test_gemm_f32x3_gpu.py holds them to it).
+// Error against 64 bits, relative 2-norm, random operands of both signs, by FMA (gemm_f32.cu) and here: K 256 1.49e-7 and 8.0e-8, 2,048
+// 1.66e-7 and 9.8e-8, 11,008 2.24e-7 and 1.46e-7.  Sums of one sign collect what is cut off: 6.0e-8 and 7.1e-8 at K 512, 7.0e-8 and
+// 7.3e-8 at 2,048, 1.33e-7 and 1.08e-7 at 11,008.  Twice the chunk would save the drain half its work and is no longer the nearer one there.
 // A result that is not finite (an infinite or not-a-number operand has no three parts; a part may round up to infinity) is
 // computed again by plain FMA.
 //

@@ -1,7 +1,7 @@
 // What a step's host side does with Python's lists: their numbers go into the int32 arrays that the kernels read.  numpy and array
 // take 25 to 35 ns a number (4,131 earlier tokens of sixteen chat requests: 147 us of a 227 us draw), this loop 4.
 //
-// Called through ctypes.PyDLL, so with the interpreter's lock held; the three functions of its C interface that are needed are
+// Called through ctypes.PyDLL, so with the interpreter's lock held; the functions of its C interface that are needed are
 // declared here, so that the library builds without Python's headers and works with the interpreter that loads it.
 #include <limits.h>
 #include <stddef.h>
