@@ -17,7 +17,7 @@
 // large batch: mma.sync and tcgen05.mma give the same bits for the same 16 k (test_gemm_f32x3_gpu.py holds them to it).
 // Error against 64 bits, relative 2-norm, random operands of both signs, by FMA (gemm_f32.cu) and here: K 256 1.49e-7 and 8.0e-8, 2,048
 // 1.66e-7 and 9.8e-8, 11,008 2.24e-7 and 1.46e-7.  Sums of one sign collect what is cut off: 6.0e-8 and 7.1e-8 at K 512, 7.0e-8 and
-// 7.3e-8 at 2,048, 1.33e-7 and 1.08e-7 at 11,008.  Twice the chunk would save the drain half its work and is no longer the nearer one there.
+// 7.3e-8 at 2,048, 1.33e-7 and 1.08e-7 at 11,008.
 // A result that is not finite (an infinite or not-a-number operand has no three parts; a part may round up to infinity) is
 // computed again by plain FMA.
 //
