@@ -106,7 +106,8 @@ __device__ __forceinline__ void f3_tma_3d_once(unsigned dst, const CUtensorMap* 
 // the 16-row side of mma.sync m16n8k16, the rows of x its 8 columns (two such tiles for 9 to 16 rows), and a thread's 16 bytes
 // of a row fill its four k slots (the sum over 16 k has no order).  A chunk takes some 700 cycles, its 12 MMAs waiting for one
 // another, so it takes many warps to keep up with the copies.  The warp of a block's second half adds its chunks to the first
-// half's sum, in shared memory, where one more warp adds the blocks.
+// half's sum, in shared memory, where one more warp adds the blocks.  It waits for that sum at an mbarrier (`half_done`), like every
+// wait here with a limit: at a hardware barrier it would wait for good once a warp has given up.
 // Measured, us for 1 / 8 / 16 rows: 151,936 features x 2,048 180 / 195 / 265 (6.9 TB/s; by FMA 176 / 230 / 440), 22,016 x 2,048
 // 32 / 35 / 47 (27 / 40 / 71), 2,048 x 11,008 19 / 20 / 28 (16 / 25 / 41): the end of a product, when the last stages' chunks are
 // on their way, is longer than by FMA.  Two warps a stage: 35, 21; stages of 256 k: 39, 23; sixteen warps with a chunk each of every
@@ -123,7 +124,7 @@ template <int MP> struct F3Rows {                // MP: rows of x in a stage
   static constexpr int RED = 2 * F3R_FEATURES * MP;             // floats of one slot of block values
   static constexpr int WARPS = STAGES * 4;
   static constexpr int THREADS = (WARPS + 2) * 32;
-  static constexpr int SMEM = 1024 + STAGES * (STAGE + RED * 4) + STAGES * 4 * 8;
+  static constexpr int SMEM = 1024 + STAGES * (STAGE + RED * 4) + STAGES * 6 * 8;
 };
 
 __device__ __forceinline__ void f3_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
@@ -145,6 +146,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   unsigned long long* empty = full + S;
   unsigned long long* red_full = empty + S;
   unsigned long long* red_empty = red_full + S;
+  unsigned long long* half_done = red_empty + S;                 // two of each stage, one a block
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int spans = (K + F3R_K - 1) / F3R_K, groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
   const int items = ((groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * spans;
@@ -155,6 +157,8 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       mbar_init(empty + s, 4);
       mbar_init(red_full + s, 2);
       mbar_init(red_empty + s, 1);
+      mbar_init(half_done + 2 * s, 1);
+      mbar_init(half_done + 2 * s + 1, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -233,7 +237,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   // MMA row g of the 16 is feature (g mod 2) * 4 + g / 2 of the group, and row g + 8 that + 8: the two rows whose 64 bytes a warp reads
   // together then lie in different halves of the banks.
   const int s = warp >> 2, block = (warp >> 1) & 1, half = warp & 1, g = lane >> 2, t = lane & 3, f = (g & 1) * 4 + (g >> 1);
-  const int pair = 1 + (warp >> 1);                              // the named barrier of a block's two warps
+  unsigned long long* first_half = half_done + 2 * s + block;
   bool ok = true;
   unsigned parity = 0;
   const unsigned line0 = (block * F3_BLOCK_CHUNKS + half * 4) * 128;
@@ -285,7 +289,12 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
       __syncwarp();
     } else {
-      asm volatile("bar.sync %0, 64;\n" ::"r"(pair) : "memory");
+      // within one phase: the first half comes again only behind red_empty, so behind this warp's red_full
+      if (ok) {
+        ok = mbar_wait(first_half, parity);
+        if (!ok && lane == 0) atomicExch(err, 59);
+      }
+      __syncwarp();
     }
 #pragma unroll
     for (int n = 0; n < TILES; ++n)
@@ -299,12 +308,8 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         sum += v[2][n][e];
         *at = sum + v[3][n][e];
       }
-    if (half == 0) {
-      asm volatile("bar.arrive %0, 64;\n" ::"r"(pair) : "memory");
-    } else {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(red_full + s);
-    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(half == 0 ? first_half : red_full + s);
   }
 }
 
