@@ -99,6 +99,13 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
   }
   return false;
 }
+// The last thing a thread does that filled a ring of `stages`: its `issued` copies have landed when it returns (or the limit has passed), so
+// that none of them writes into shared memory that a later CTA already has.  Readers that take everything have waited for them anyway;
+// readers that gave up have not.
+__device__ __forceinline__ void mbar_landed(unsigned long long* full, int stages, int issued) {
+  bool ok = true;
+  for (int i = issued > stages ? issued - stages : 0; i < issued && ok; ++i) ok = mbar_wait(full + i % stages, (unsigned)(i / stages) & 1);
+}
 // One contiguous piece of global memory into shared memory (both 16-byte aligned, a multiple of 16
 // bytes); the bytes are counted on the mbarrier.
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {

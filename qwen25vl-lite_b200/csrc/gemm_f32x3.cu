@@ -169,7 +169,6 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     // ---- producer ----
     if (lane == 0) {
       const unsigned long long once = l2_evict_first();
-      bool ok = true;
       auto weights = [&](int item) {
         const int s = item % S, g = (int)blockIdx.x + item / spans * (int)gridDim.x, line = item % spans * (F3R_K / 32);
         mbar_expect_tx(full + s, Shape::STAGE);
@@ -184,14 +183,13 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       for (int i = 0; i < ahead; ++i) weights(i);
       pdl_wait();
       for (int i = 0; i < ahead; ++i) rows(i);
-      for (int i = ahead; i < items; ++i) {
-        if (ok) {
-          ok = mbar_wait(empty + i % S, (unsigned)(i / S - 1) & 1);
-          if (!ok) { atomicExch(err, 51); break; }               // nobody reads what was not asked for: the readers give up too
-        }
-        weights(i);
-        rows(i);
+      int issued = ahead;
+      for (; issued < items; ++issued) {
+        if (!mbar_wait(empty + issued % S, (unsigned)(issued / S - 1) & 1)) { atomicExch(err, 51); break; }      // nobody reads what was not asked for: the readers give up too
+        weights(issued);
+        rows(issued);
       }
+      mbar_landed(full, S, issued);
     }
     return;
   }
@@ -470,11 +468,14 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
   bool ok = true;
 
   if (warp == W_WARP) {
-    if (lane == 0)
-      for (int it = ahead; it < mine; ++it) {
+    if (lane == 0) {
+      int it = ahead;
+      for (; it < mine; ++it) {
         if (!mbar_wait(w_empty + it % WS, (unsigned)(it / WS - 1) & 1)) { atomicExch(err, 55); break; }
         load_w(it);
       }
+      mbar_landed(w_full, WS, it);
+    }
   } else if (warp == X_WARP) {
     if (lane == 0) {
       int xt = 0;
@@ -488,6 +489,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
           mbar_expect_tx(x_full + s, Shape::XSTAGE);
           f3_tma_3d(smem_u32(xring + s * Shape::XSTAGE), &map_p, c * F3_CHUNK, tile % row_tiles * BN, 0, x_full + s);
         }
+      mbar_landed(x_full, XS, xt);
     }
   } else if (warp == MMA_WARP) {
     // The whole warp walks, in uniform registers, and one lane issues: a lane that walks alone moves every operand into them,
@@ -524,6 +526,8 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
         __syncwarp();
         if (x_done && ++xs == XS) { xs = 0; x_parity ^= 1; }
       }
+    // the last commit stands for all products asked for: none of them still runs when tensor memory goes back
+    if (it > 0) mbar_wait(done + ((it - 1) & 1), (unsigned)((it - 1) >> 1) & 1);
   } else if (warp >= Shape::DRAINS) {
     // ---- converters ----
     const int set = (warp - Shape::DRAINS) >> 2, quarter = warp & 3, row = quarter * 32 + lane;

@@ -28,3 +28,29 @@ def test_every_wait_on_an_mbarrier_goes_through_the_bounded_one():
     for name in SOURCES:
         found = re.findall(r"mbarrier\.(?:try_wait|test_wait)", _code(name))
         assert len(found) == (1 if name == "common.cuh" else 0), name
+
+
+def _kernels(name):
+    """(kernel, body) of a source file."""
+    code = _code(name)
+    for m in re.finditer(r"__global__ void[^{;]*?(\w+_kernel)\(", code):
+        at = code.index("{", code.index(")", m.end()))
+        depth, end = 1, at + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(code[end], 0)
+            end += 1
+        yield m.group(1), code[at:end]
+
+
+@pytest.mark.parametrize("name", ["gemm_f32x3.cu"])
+def test_copies_have_landed_before_a_kernel_ends(name):
+    """Where readers give up, copies may still be on their way: each ring's producer waits for its own last ones, and the thread that
+    issues products for its own last commit, before shared and tensor memory go to another CTA."""
+    rings = {"f3_rows_kernel": ["full"], "f3_tile_kernel": ["w_full", "x_full"]}
+    found = dict(_kernels(name))
+    assert set(rings) <= set(found)
+    for kernel, body in found.items():
+        assert re.findall(r"mbar_landed\((\w+),", body) == rings.get(kernel, [])
+        if "tc5_mma" in body:
+            last = body.index("mbar_wait(done + ((it - 1) & 1)")
+            assert body.rindex("tc5_commit(") < last < body.index("tcgen05.dealloc")
