@@ -19,7 +19,7 @@
 // 1.66e-7 and 9.8e-8, 11,008 2.24e-7 and 1.46e-7.  Sums of one sign collect what is cut off: 6.0e-8 and 7.1e-8 at K 512, 7.0e-8 and
 // 7.3e-8 at 2,048, 1.33e-7 and 1.08e-7 at 11,008.
 // A result that is not finite (an infinite or not-a-number operand has no three parts; a part may round up to infinity) is
-// computed again by plain FMA.
+// computed again by plain FMA, behind its CTA's pipeline.
 //
 //   * up to 16 rows (decode steps): f3_rows_kernel, a stream of the weights, mma.sync;
 //   * more rows: f3_parts_kernel cuts A into its three parts, f3_tile_kernel multiplies, tcgen05; where its tiles are too few
@@ -63,25 +63,90 @@ __device__ __forceinline__ ulonglong2 f3_lds(unsigned addr) {
 }
 __device__ __forceinline__ bool f3_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
 
-// A result by plain FMA, in the order of gemm_f32.cu.
-__device__ __noinline__ float f3_plain(const float* __restrict__ a, const float* __restrict__ w, int K) {
-  float total = 0.f;
-  for (int k0 = 0; k0 < K; k0 += 128) {
-    float even = 0.f, odd = 0.f;
-    for (int k = k0; k < min(K, k0 + 128); k += 2) {
-      even = fmaf(a[k], w[k], even);
-      odd = fmaf(a[k + 1], w[k + 1], odd);
-    }
-    total += even + odd;
+// ---- results that are not finite --------------------------------------------------------------------------------------
+// They are marked where they are stored and computed again when their CTA's pipeline has ended: a dot product of 11,008 terms takes
+// some microseconds, during which warps with bounded waits would stand.
+//
+// Four dot products of a row by plain FMA, by a warp: lane l has k = 4 l .. 4 l + 3 of every 128, in one chain; one order, like all here.
+template <int STEPS>
+__device__ __forceinline__ void f3_plain_steps(const float* a, const float* const (&w)[4], float (&sum)[4]) {      // STEPS x 128 k; all loads first
+  float x[STEPS][4];                             // perhaps not aligned
+  float4 v[STEPS][4];
+#pragma unroll
+  for (int t = 0; t < STEPS; ++t) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[t][j] = __ldcg(reinterpret_cast<const float4*>(w[j] + t * 128));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[t][j] = __ldcg(a + t * 128 + j);
   }
-  return total;
+#pragma unroll
+  for (int t = 0; t < STEPS; ++t)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      sum[j] = fmaf(x[t][3], v[t][j].w, fmaf(x[t][2], v[t][j].z, fmaf(x[t][1], v[t][j].y, fmaf(x[t][0], v[t][j].x, sum[j]))));
 }
-// The results of rows m .. end of a feature that are not finite, computed again.
-__device__ __noinline__ void f3_again(const float* A, const float* W, float* C, int m, int end, int n, int K, int lda, int ldw, int ldc, float more) {
-  for (; m < end; ++m) {
-    float* c = C + (size_t)m * ldc + n;
-    if (!f3_finite(*c)) *c = f3_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K) + more;
+__device__ __forceinline__ void f3_plain(const float* a, const float* const (&row)[4], int K, float (&sum)[4]) {
+  int k = (threadIdx.x & 31) * 4;
+  const float* w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    sum[j] = 0.f;
+    w[j] = row[j] + k;
   }
+  a += k;
+  auto on = [&](int by) {
+    k += by;
+    a += by;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] += by;
+  };
+  for (; k + 128 < K; on(256)) f3_plain_steps<2>(a, w, sum);
+  if (k < K) f3_plain_steps<1>(a, w, sum);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) sum[j] = warp_sum(sum[j]);
+}
+// All warps of a CTA look at rows m0 .. m0 + rows of features n0 .. n1 (`marks`: a word of shared memory for each 32 features of a row), and
+// four features of a row are computed again by a warp.  A row of A that holds a NaN has nothing else to become, and shows it early where all
+// of it is NaN: the products after activations that have all turned into NaN take little longer (1,500 rows x 22,016 x 2,048
+// 572 -> 646 us, one row 39 -> 47; with one infinity among the 1,500 rows 1,223 us).
+__device__ __noinline__ void f3_again(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* C,
+                                      unsigned* marks, int m0, int rows, int n0, int n1, int K, int lda, int ldw, int ldc) {
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5, lane = threadIdx.x & 31, words = (n1 - n0 + 31) / 32;
+  bool any = false;
+  for (int r = warp; r < rows; r += warps) {
+    const float* a = A + (size_t)(m0 + r) * lda;
+    bool looked = false, nan = false;
+    for (int i = 0; i < words; ++i) {
+      const int n = n0 + i * 32 + lane;
+      unsigned mark = nan ? 0 : __ballot_sync(0xffffffffu, n < n1 && !f3_finite(__ldcg(C + (size_t)(m0 + r) * ldc + min(n, n1 - 1))));
+      for (int k = lane; mark != 0 && !looked && !nan && k < K; k += 128) {      // K is a multiple of 32: the lanes go together
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (k + 32 * j < K) nan |= isnan(__ldcg(a + k + 32 * j));
+        nan = __any_sync(0xffffffffu, nan);
+      }
+      looked |= mark != 0;
+      if (nan) mark = 0;
+      any |= mark != 0;
+      if (lane == 0) marks[r * words + i] = mark;
+    }
+  }
+  if (__syncthreads_or(any)) {
+    for (int u = warp; u < rows * words * 8; u += warps) {
+      const unsigned mark = marks[u >> 3] >> (u & 7) * 4 & 15;
+      if (mark == 0) continue;
+      const int m = m0 + (u >> 3) / words, n = n0 + (u >> 3) % words * 32 + (u & 7) * 4;
+      const float* w[4];
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = W + (size_t)min(n + j, n1 - 1) * ldw;
+      f3_plain(A + (size_t)m * lda, w, K, v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (lane == j && (mark >> j & 1)) C[(size_t)m * ldc + n + j] = v[j] + (bias ? bias[n + j] : 0.f);
+    }
+  }
+  __syncthreads();                                               // the marks are free
 }
 
 __device__ __forceinline__ void f3_tma_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
@@ -124,7 +189,7 @@ template <int MP> struct F3Rows {                // MP: rows of x in a stage
   static constexpr int RED = 2 * F3R_FEATURES * MP;             // floats of one slot of block values
   static constexpr int WARPS = STAGES * 4;
   static constexpr int THREADS = (WARPS + 2) * 32;
-  static constexpr int SMEM = 1024 + STAGES * (STAGE + RED * 4) + STAGES * 6 * 8;
+  static constexpr int SMEM = 1024 + STAGES * (STAGE + RED * 4) + STAGES * 6 * 8 + 16;
 };
 
 __device__ __forceinline__ void f3_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
@@ -147,6 +212,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   unsigned long long* red_full = empty + S;
   unsigned long long* red_empty = red_full + S;
   unsigned long long* half_done = red_empty + S;                 // two of each stage, one a block
+  int* odd = reinterpret_cast<int*>(half_done + 2 * S);          // a result is not finite
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int spans = (K + F3R_K - 1) / F3R_K, groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
   const int items = ((groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * spans;
@@ -160,6 +226,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       mbar_init(half_done + 2 * s, 1);
       mbar_init(half_done + 2 * s + 1, 1);
     }
+    *odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
@@ -191,9 +258,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
       mbar_landed(full, S, issued);
     }
-    return;
-  }
-  if (warp == Shape::WARPS + 1) {
+  } else if (warp == Shape::WARPS + 1) {
     // ---- the blocks' values, added in order ----
     constexpr int V = (F3R_FEATURES * MP + 31) / 32;
     pdl_wait();                                                  // the kernel before may still read what this one overwrites
@@ -221,16 +286,15 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         for (int v = 0; v < V; ++v) {
           const int m = v * 2 + (lane >> 4);
           if (m < M && n < N) {
-            if (!f3_finite(total[v])) total[v] = f3_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
-            C[(size_t)m * ldc + n] = total[v] + (bias ? bias[n] : 0.f);
+            const float value = total[v] + (bias ? bias[n] : 0.f);
+            C[(size_t)m * ldc + n] = value;
+            if (!f3_finite(value)) *odd = 1;
           }
           total[v] = 0.f;
         }
       }
     }
-    return;
-  }
-
+  } else {
   // ---- four warps, one stage ----
   // MMA row g of the 16 is feature (g mod 2) * 4 + g / 2 of the group, and row g + 8 that + 8: the two rows whose 64 bytes a warp reads
   // together then lie in different halves of the banks.
@@ -308,6 +372,13 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     __syncwarp();
     if (lane == 0) mbar_arrive(half == 0 ? first_half : red_full + s);
+  }
+  }
+  // every warp gets here: all waits are bounded
+  __syncthreads();
+  if (*odd != 0) {
+    for (int g = blockIdx.x; g < groups; g += gridDim.x)
+      f3_again(A, W, bias, C, reinterpret_cast<unsigned*>(smem), 0, M, g * F3R_FEATURES, min(N, (g + 1) * F3R_FEATURES), K, lda, ldw, ldc);
   }
 }
 
@@ -423,6 +494,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
   // of each of the two buffers (a stage of W's parts and an accumulator): both are free for the MMAs; these have ended
   unsigned long long *ready = x_empty + XS, *done = ready + 2;
   unsigned* tmem_at = reinterpret_cast<unsigned*>(done + 2);
+  int* odd = reinterpret_cast<int*>(tmem_at + 1);                // a result is not finite
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int W_WARP = Shape::DRAINS + 4 * SETS, X_WARP = W_WARP + 1, MMA_WARP = W_WARP + 2;
   const int row_tiles = (M + BN - 1) / BN, tiles = row_tiles * ((N + 127) / 128);
@@ -440,6 +512,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
       mbar_init(ready + b, 4 + Shape::DRAINS);
       mbar_init(done + b, 1);
     }
+    *odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
@@ -607,11 +680,12 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
           bool finite = true;
 #pragma unroll
           for (int j = 0; j < WIDTH; ++j, dst += pitch) {
-            finite &= f3_finite(acc[j]);
-            if (m0 + j < M) *dst = acc[j] + more;
+            const float value = acc[j] + more;
+            finite &= f3_finite(value);
+            if (m0 + j < M) *dst = value;
             asm volatile("" : "+l"(dst));        // one address after the other: all of them at once do not fit the registers
           }
-          if (whole && !finite) f3_again(A, W, C, m0, min(M, m0 + WIDTH), n, K, lda, ldw, ldc, more);
+          if (whole && !finite) *odd = 1;
         }
         __syncwarp();
 #pragma unroll
@@ -628,6 +702,11 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
     tc5_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(512) : "memory");
   }
+  if (*odd != 0)
+    for (int tile = first_tile; tile < tiles; tile += step) {
+      const int m0 = tile % row_tiles * BN, n0 = tile / row_tiles * 128;
+      f3_again(A, W, bias, C, reinterpret_cast<unsigned*>(xring), m0, min(BN, M - m0), n0, min(N, n0 + 128), K, lda, ldw, ldc);
+    }
 }
 
 // The planes of a split product, block by block, + bias; a thread has one element of the output.
@@ -636,9 +715,11 @@ f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, con
               float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
   pdl_trigger();
   pdl_wait();
+  __shared__ unsigned marks[8];
   const size_t size = (size_t)M * N;
   const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK;
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < size; i += (size_t)gridDim.x * 256) {
+  for (size_t i0 = (size_t)blockIdx.x * 256; i0 < size; i0 += (size_t)gridDim.x * 256) {
+    const size_t i = min(i0 + threadIdx.x, size - 1);
     const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
     float total = 0.f;
     for (int b0 = 0; b0 < blocks; b0 += 8) {     // eight loads on their way at a time
@@ -648,8 +729,15 @@ f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, con
 #pragma unroll
       for (int j = 0; j < 8; ++j) total = b0 + j < blocks ? total + v[j] : total;
     }
-    if (!f3_finite(total)) total = f3_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
-    C[(size_t)m * ldc + n] = total + (bias ? bias[n] : 0.f);
+    total += bias ? bias[n] : 0.f;
+    if (i0 + threadIdx.x < size) C[(size_t)m * ldc + n] = total;
+    if (__syncthreads_or(!f3_finite(total)))
+      for (size_t at = i0, end = min(i0 + 256, size); at < end;) {        // row by row
+        const int row = (int)(at / N);
+        const size_t begin = (size_t)row * N, stop = min(end, begin + N);
+        f3_again(A, W, bias, C, marks, row, 1, (int)(at - begin), (int)(stop - begin), K, lda, ldw, ldc);
+        at = stop;
+      }
   }
 }
 

@@ -67,3 +67,37 @@ def test_rows_beyond_the_scratch_limit(monkeypatch):
     whole = _product(a, w, b)
     monkeypatch.setattr(kernels, "F32X3_SCRATCH", 1)
     assert torch.equal(_product(a, w, b), whole)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 5000, 11008), (16, 5000, 2048), (64, 2048, 11008), (300, 20000, 2048), (300, 2000, 18944)])
+def test_rows_that_are_not_numbers(m, n, k):
+    """Activations that have all turned into NaN, and rows that hold an infinity: computed again behind the pipeline, so that no wait in it
+    runs out, and in a time of the same order."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, w = torch.randn(m, k, generator=gen, device="cuda"), torch.randn(n, k, generator=gen, device="cuda")
+    out = torch.empty(m, n, device="cuda")
+    from qwen25vl_lite.ops import kernels
+
+    def least(x):
+        times = []
+        for _ in range(4):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(200_000)                       # the call is queued before the GPU begins it
+            start.record()
+            kernels.gemm_f32(x, w, None, out, fixed=True)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        assert int(kernels.error_flag(out.device)) == 0
+        return min(times)
+
+    clean = least(a)
+    assert bool(out.isfinite().all())
+    whole = out.clone()
+    assert least(torch.full_like(a, float("nan"))) < 4 * clean + 0.02
+    assert bool(out.isnan().all())
+    a[m // 2, k - 1] = float("inf")
+    least(a)
+    assert torch.equal(out[m // 2], w[:, k - 1].sign() * float("inf"))
+    rest = [i for i in range(m) if i != m // 2]
+    assert torch.equal(out[rest], whole[rest])
