@@ -709,17 +709,17 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
     }
 }
 
-// The planes of a split product, block by block, + bias; a thread has one element of the output.
-__global__ void __launch_bounds__(256)
+// The planes of a split product, block by block, + bias; a thread has one element of the output.  Results that are not finite are
+// computed again by their warp, one after the other, with few registers (f3_again's would leave three CTAs of this kernel to an SM).
+__global__ void __launch_bounds__(256, 6)
 f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
               float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
   pdl_trigger();
   pdl_wait();
-  __shared__ unsigned marks[8];
   const size_t size = (size_t)M * N;
-  const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK;
-  for (size_t i0 = (size_t)blockIdx.x * 256; i0 < size; i0 += (size_t)gridDim.x * 256) {
-    const size_t i = min(i0 + threadIdx.x, size - 1);
+  const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK, lane = threadIdx.x & 31;
+  for (size_t i0 = (size_t)blockIdx.x * 256 + (threadIdx.x & ~31); i0 < size; i0 += (size_t)gridDim.x * 256) {       // a warp has 32 of them
+    const size_t i = min(i0 + lane, size - 1);
     const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
     float total = 0.f;
     for (int b0 = 0; b0 < blocks; b0 += 8) {     // eight loads on their way at a time
@@ -729,15 +729,28 @@ f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, con
 #pragma unroll
       for (int j = 0; j < 8; ++j) total = b0 + j < blocks ? total + v[j] : total;
     }
-    total += bias ? bias[n] : 0.f;
-    if (i0 + threadIdx.x < size) C[(size_t)m * ldc + n] = total;
-    if (__syncthreads_or(!f3_finite(total)))
-      for (size_t at = i0, end = min(i0 + 256, size); at < end;) {        // row by row
-        const int row = (int)(at / N);
-        const size_t begin = (size_t)row * N, stop = min(end, begin + N);
-        f3_again(A, W, bias, C, marks, row, 1, (int)(at - begin), (int)(stop - begin), K, lda, ldw, ldc);
-        at = stop;
+    const float more = bias ? bias[n] : 0.f;
+    total += more;
+    for (unsigned todo = __ballot_sync(0xffffffffu, !f3_finite(total)); todo != 0; todo &= todo - 1) {
+      const int from = __ffs(todo) - 1;
+      const float* a = A + (size_t)__shfl_sync(0xffffffffu, m, from) * lda;
+      const float* w = W + (size_t)__shfl_sync(0xffffffffu, n, from) * ldw;
+      float sum = 0.f;                           // as f3_plain has it
+      bool nan = false;                          // the row holds one: nothing else can come of it
+      for (int k0 = 0; k0 < K && !nan; k0 += 128) {
+        const int k = k0 + lane * 4;
+        if (k < K) {
+          const float x0 = __ldcg(a + k), x1 = __ldcg(a + k + 1), x2 = __ldcg(a + k + 2), x3 = __ldcg(a + k + 3);
+          const float4 v = __ldcg(reinterpret_cast<const float4*>(w + k));
+          sum = fmaf(x3, v.w, fmaf(x2, v.z, fmaf(x1, v.y, fmaf(x0, v.x, sum))));
+          nan = isnan(x0) || isnan(x1) || isnan(x2) || isnan(x3);
+        }
+        nan = __any_sync(0xffffffffu, nan);
       }
+      sum = warp_sum(sum) + more;
+      if (lane == from && !nan) total = sum;
+    }
+    if (i0 + lane < size) C[(size_t)m * ldc + n] = total;
   }
 }
 
