@@ -39,20 +39,20 @@ __device__ __forceinline__ unsigned f3_pack(float lo, float hi) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
-__device__ __forceinline__ f32x2 f3_less(f32x2 x, unsigned part) {       // what a part leaves
-  f32x2 r;
-  asm("{\n .reg .b32 a, b;\n .reg .b64 p;\n shl.b32 a, %2, 16;\n and.b32 b, %2, 0xffff0000;\n mov.b64 p, {a, b};\n"
-      " sub.rn.f32x2 %0, %1, p;\n}\n" : "=l"(r) : "l"(x), "r"(part));
+// What a part leaves: number - part, exact.  (The mixed FMA reads the part as it is packed: a pair of numbers is cut up in 10 cycles of
+// a scheduler, 12 where the parts are unpacked for a packed subtraction.)
+__device__ __forceinline__ float2 f3_less(float2 x, unsigned part) {
+  float2 r;
+  asm("{\n .reg .b16 a, b, m;\n mov.b32 {a, b}, %2;\n mov.b16 m, 0xbf80;\n"           // m = -1
+      " fma.rn.f32.bf16 %0, a, m, %3;\n fma.rn.f32.bf16 %1, b, m, %4;\n}\n" : "=f"(r.x), "=f"(r.y) : "r"(part), "f"(x.x), "f"(x.y));
   return r;
 }
 __device__ __forceinline__ void f3_split(f32x2 x, unsigned& hi, unsigned& mid, unsigned& lo) {
   float2 v = split2(x);
   hi = f3_pack(v.x, v.y);
-  x = f3_less(x, hi);
-  v = split2(x);
+  v = f3_less(v, hi);
   mid = f3_pack(v.x, v.y);
-  x = f3_less(x, mid);
-  v = split2(x);
+  v = f3_less(v, mid);
   lo = f3_pack(v.x, v.y);
 }
 
@@ -167,29 +167,36 @@ __device__ __forceinline__ void f3_tma_3d_once(unsigned dst, const CUtensorMap* 
 // One persistent CTA per SM; its items are (group of 16 features, 512 k), one stage of the ring each, which two copies fill: a
 // box of 16 rows of W and one of the rows of x (the copy engine takes a request about every 90 cycles whatever its size).  K is
 // seen as lines of 32; a row of W's box holds 17 of them, the last one not used, so that the 128-byte swizzle puts the same
-// line of eight rows into eight different bank groups.  Four warps share a stage, half a block each: the weights are
+// line of eight rows into eight different bank groups.  A team of four warps has an item, half a block a warp: the weights are
 // the 16-row side of mma.sync m16n8k16, the rows of x its 8 columns (two such tiles for 9 to 16 rows), and a thread's 16 bytes
-// of a row fill its four k slots (the sum over 16 k has no order).  A chunk takes some 700 cycles, its 12 MMAs waiting for one
-// another, so it takes many warps to keep up with the copies.  The warp of a block's second half adds its chunks to the first
-// half's sum, in shared memory, where one more warp adds the blocks.  It waits for that sum at an mbarrier (`half_done`), like every
-// wait here with a limit: at a hardware barrier it would wait for good once a warp has given up.
-// Measured, us for 1 / 8 / 16 rows: 151,936 features x 2,048 180 / 195 / 265 (6.9 TB/s; by FMA 176 / 230 / 440), 22,016 x 2,048
-// 32 / 35 / 47 (27 / 40 / 71), 2,048 x 11,008 19 / 20 / 28 (16 / 25 / 41): the end of a product, when the last stages' chunks are
-// on their way, is longer than by FMA.  Two warps a stage: 35, 21; stages of 256 k: 39, 23; sixteen warps with a chunk each of every
-// stage, which is free at once: 37, 22 (every warp pays for every stage's barriers).
+// of a row fill its four k slots (the sum over 16 k has no order).
+// Up to 4 rows leave columns idle, and cutting numbers into parts is what a warp spends most on: there the columns are the rows of 2 or
+// 4 lines side by side, cut up once, of which the MMAs of a line use their own; a warp works on two lines at a time, as the 12 MMAs of a chunk wait
+// for one another; and every chunk's value goes to the warp that adds the blocks.  With more rows the warp of a block's second half adds its chunks to the
+// first half's sum, in shared memory; it waits for that sum at an mbarrier (`half_done`), like every wait here with a limit: at a
+// hardware barrier it would wait for good once a warp has given up.
+// Measured, us for 1 / 2 / 4 / 8 / 16 rows (in a row of launches over weights that are not in L2), by FMA in brackets: 22,016 features x 2,048
+// 27.4 / 28.4 / 28.8 / 30.6 / 44.5 (26.7 / 27.7 / 30.9 / 39.4 / 70.4), 2,048 x 11,008 16.2 / 17.6 / 17.8 / 18.5 / 26.5 (15.2 / 16.0 / 18.3 / 24.9 / 41),
+// 2,560 x 2,048 6.7 / 6.7 / 7.0 / 6.9 / 10.7 (5.0 / 5.5 / 6.5 / 8.6 / 15.8), 320 x 256 2.3 / 2.3 / 2.2 / 2.6 / 3.4 (2.2 / 2.2 / 2.5 / 3.4 / 3.6).
+// One and two rows stay behind FMA where the first stages arrive together: cutting up 32 KB takes four schedulers some 320 cycles, with every
+// team's 12 MMAs behind it.  Each line's rows cut up for itself, one line at a time, three quarters of an item's divisions by the number
+// of spans: 30.2, 18.7, 7.5 us for one row.  Two warps a stage: 35, 21; stages of 256 k: 39, 23; sixteen warps with a chunk each of every
+// stage: 37, 22; two teams of eight warps with two lines each: 32, 20; lines as the MMA's rows and items of 4 features x 2,048 k, the rows
+// in shared memory whole: 28.3, 17.0, but 15.3 for 4,608 x 3,584 (12.4).
 #define F3R_FEATURES 16
 #define F3R_K 512
 #define F3R_PITCH (17 * 128)                     // bytes between the rows of W in a stage
 #define F3R_W_BYTES (F3R_FEATURES * F3R_PITCH)
 
-template <int MP> struct F3Rows {                // MP: rows of x in a stage
+template <int MP, int TEAMS> struct F3Rows {     // MP: rows of x in a stage; teams of four warps
   static constexpr int TILES = MP > 8 ? 2 : 1;
   static constexpr int STAGE = F3R_W_BYTES + MP * F3R_K * 4;
-  static constexpr int STAGES = MP <= 4 ? 5 : MP == 8 ? 4 : 3;
-  static constexpr int RED = 2 * F3R_FEATURES * MP;             // floats of one slot of block values
-  static constexpr int WARPS = STAGES * 4;
-  static constexpr int THREADS = (WARPS + 2) * 32;
-  static constexpr int SMEM = 1024 + STAGES * (STAGE + RED * 4) + STAGES * 6 * 8 + 16;
+  static constexpr int STAGES = MP == 1 ? 6 : MP <= 4 ? 5 : MP == 8 ? 4 : 3;
+  static constexpr int VALUES = MP < 8 ? F3_BLOCK_CHUNKS : 1;    // that a team leaves of a block: its chunks', or their sum
+  static constexpr int RED = F3R_K / F3_BLOCK * VALUES * F3R_FEATURES * MP;          // floats that a team leaves
+  static constexpr int THREADS = (TEAMS * 4 + 2) * 32;
+  static constexpr int SMEM = 1024 + STAGES * STAGE + TEAMS * RED * 4 + (2 * STAGES + 4 * TEAMS) * 8 + 16;
+  static_assert(SMEM <= 227 * 1024 && TEAMS <= STAGES, "shared memory");
 };
 
 __device__ __forceinline__ void f3_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
@@ -197,22 +204,22 @@ __device__ __forceinline__ void f3_mma(float (&c)[4], const unsigned (&a)[4], co
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-template <int MP>
-__global__ void __launch_bounds__(F3Rows<MP>::THREADS, 1)
+template <int MP, int TEAMS>
+__global__ void __launch_bounds__(F3Rows<MP, TEAMS>::THREADS, 1)
 f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const float* __restrict__ A,
                const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K, int lda, int ldw,
                int ldc, bool early, int* err) {
-  using Shape = F3Rows<MP>;
+  using Shape = F3Rows<MP, TEAMS>;
   constexpr int S = Shape::STAGES, TILES = Shape::TILES;
   extern __shared__ unsigned char f3_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)f3_raw + 1023) & ~(uintptr_t)1023);
   float* red = reinterpret_cast<float*>(smem + S * Shape::STAGE);
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(red + S * Shape::RED);
+  unsigned long long* full = reinterpret_cast<unsigned long long*>(red + TEAMS * Shape::RED);
   unsigned long long* empty = full + S;
   unsigned long long* red_full = empty + S;
-  unsigned long long* red_empty = red_full + S;
-  unsigned long long* half_done = red_empty + S;                 // two of each stage, one a block
-  int* odd = reinterpret_cast<int*>(half_done + 2 * S);          // a result is not finite
+  unsigned long long* red_empty = red_full + TEAMS;
+  unsigned long long* half_done = red_empty + TEAMS;             // two of each team, one a block
+  int* odd = reinterpret_cast<int*>(half_done + 2 * TEAMS);      // a result is not finite
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int spans = (K + F3R_K - 1) / F3R_K, groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
   const int items = ((groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * spans;
@@ -221,7 +228,9 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     for (int s = 0; s < S; ++s) {
       mbar_init(full + s, 1);
       mbar_init(empty + s, 4);
-      mbar_init(red_full + s, 2);
+    }
+    for (int s = 0; s < TEAMS; ++s) {
+      mbar_init(red_full + s, MP < 8 ? 4 : 2);
       mbar_init(red_empty + s, 1);
       mbar_init(half_done + 2 * s, 1);
       mbar_init(half_done + 2 * s + 1, 1);
@@ -232,146 +241,194 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   __syncthreads();
   pdl_trigger();
 
-  if (warp == Shape::WARPS) {
+  if (warp == TEAMS * 4) {
     // ---- producer ----
     if (lane == 0) {
       const unsigned long long once = l2_evict_first();
-      auto weights = [&](int item) {
-        const int s = item % S, g = (int)blockIdx.x + item / spans * (int)gridDim.x, line = item % spans * (F3R_K / 32);
+      // counters: a division stands between a stage that is free and its copies
+      struct { int line, n0; } w = {0, (int)blockIdx.x * F3R_FEATURES}, x = {0, 0};
+      const int end = spans * (F3R_K / 32);
+      auto weights = [&](int s) {
         mbar_expect_tx(full + s, Shape::STAGE);
-        f3_tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, line, g * F3R_FEATURES, full + s, once);
+        f3_tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.n0, full + s, once);
+        if ((w.line += F3R_K / 32) == end) w = {0, w.n0 + (int)gridDim.x * F3R_FEATURES};
       };
-      auto rows = [&](int item) {
-        const int s = item % S, line = item % spans * (F3R_K / 32);
-        f3_tma_3d(smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES, &map_x, 0, line, 0, full + s);
+      auto rows = [&](int s) {
+        f3_tma_3d(smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES, &map_x, 0, x.line, 0, full + s);
+        if ((x.line += F3R_K / 32) == end) x.line = 0;
       };
       const int ahead = min(S, items);
       if (!early) pdl_wait();
-      for (int i = 0; i < ahead; ++i) weights(i);
+      for (int s = 0; s < ahead; ++s) weights(s);
       pdl_wait();
-      for (int i = 0; i < ahead; ++i) rows(i);
-      int issued = ahead;
+      for (int s = 0; s < ahead; ++s) rows(s);
+      int issued = ahead, s = 0;
+      unsigned parity = 0;
       for (; issued < items; ++issued) {
-        if (!mbar_wait(empty + issued % S, (unsigned)(issued / S - 1) & 1)) { atomicExch(err, 51); break; }      // nobody reads what was not asked for: the readers give up too
-        weights(issued);
-        rows(issued);
+        if (!mbar_wait(empty + s, parity)) { atomicExch(err, 51); break; }       // nobody reads what was not asked for: the readers give up too
+        weights(s);
+        rows(s);
+        if (++s == S) { s = 0; parity ^= 1; }
       }
       mbar_landed(full, S, issued);
     }
-  } else if (warp == Shape::WARPS + 1) {
-    // ---- the blocks' values, added in order ----
+  } else if (warp == TEAMS * 4 + 1) {
+    // ---- the chunks' and the blocks' values, added in order ----
     constexpr int V = (F3R_FEATURES * MP + 31) / 32;
     pdl_wait();                                                  // the kernel before may still read what this one overwrites
     bool ok = true;
     float total[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) total[v] = 0.f;
+    unsigned parities = 0;                                       // a bit for each team
+    int span = 0, g = (int)blockIdx.x;
     for (int i = 0; i < items; ++i) {
-      const int s = i % S;
+      const int team = i % S % TEAMS;
       if (ok) {
-        ok = mbar_wait(red_full + s, (unsigned)(i / S) & 1);
+        ok = mbar_wait(red_full + team, parities >> team & 1);
         if (!ok && lane == 0) atomicExch(err, 52);
       }
-      const float* slot = red + s * Shape::RED;
+      parities ^= 1u << team;
+      const float* slot = red + team * Shape::RED + lane;
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+      for (int v = 0; v < V; ++v) {
+        if (V * 32 != F3R_FEATURES * MP && lane >= F3R_FEATURES * MP) continue;
 #pragma unroll
-        for (int v = 0; v < V; ++v)
-          if (V * 32 == F3R_FEATURES * MP || lane < F3R_FEATURES * MP) total[v] += slot[q * (F3R_FEATURES * MP) + v * 32 + lane];
+        for (int block = 0; block < F3R_K / F3_BLOCK; ++block) {
+          const float* at = slot + block * (Shape::VALUES * F3R_FEATURES * MP) + v * 32;
+          float sum = at[0];
+#pragma unroll
+          for (int c = 1; c < Shape::VALUES; ++c) sum += at[c * (F3R_FEATURES * MP)];
+          total[v] += sum;
+        }
+      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(red_empty + s);
-      if (i % spans == spans - 1) {
-        const int n = ((int)blockIdx.x + i / spans * (int)gridDim.x) * F3R_FEATURES + (lane & 15);
+      if (lane == 0) mbar_arrive(red_empty + team);
+      if (++span == spans) {
+        const int n = g * F3R_FEATURES + (lane & 15);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
           const int m = v * 2 + (lane >> 4);
-          if (m < M && n < N) {
+          if (m < M && n < N && (MP > 1 || lane < F3R_FEATURES)) {
             const float value = total[v] + (bias ? bias[n] : 0.f);
             C[(size_t)m * ldc + n] = value;
             if (!f3_finite(value)) *odd = 1;
           }
           total[v] = 0.f;
         }
+        span = 0;
+        g += (int)gridDim.x;
       }
     }
   } else {
-  // ---- four warps, one stage ----
+  // ---- a team's warps: four lines of its item each, half a block ----
   // MMA row g of the 16 is feature (g mod 2) * 4 + g / 2 of the group, and row g + 8 that + 8: the two rows whose 64 bytes a warp reads
   // together then lie in different halves of the banks.
-  const int s = warp >> 2, block = (warp >> 1) & 1, half = warp & 1, g = lane >> 2, t = lane & 3, f = (g & 1) * 4 + (g >> 1);
-  unsigned long long* first_half = half_done + 2 * s + block;
-  bool ok = true;
-  unsigned parity = 0;
-  const unsigned line0 = (block * F3_BLOCK_CHUNKS + half * 4) * 128;
-  const unsigned wa = smem_u32(smem + s * Shape::STAGE) + f * F3R_PITCH + line0;
-  const unsigned xa = smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES + (g & (MP < 8 ? MP - 1 : 7)) * (F3R_K * 4) + line0 + t * 16;
-  float* slot = red + s * Shape::RED + block * (F3R_FEATURES * MP) + f;
+  constexpr int SHARE = MP >= 8 ? 1 : MP == 4 ? 2 : 4;           // lines whose parts of x lie side by side
+  const int team = warp >> 2, line0 = (warp & 3) * 4, block = (warp >> 1) & 1, half = warp & 1, g = lane >> 2, t = lane & 3, f = (g & 1) * 4 + (g >> 1);
+  const unsigned wa = smem_u32(smem) + f * F3R_PITCH + line0 * 128;
+  const unsigned xa = smem_u32(smem) + F3R_W_BYTES + (g % MP & 7) * (F3R_K * 4) + (line0 + g / MP % SHARE) * 128 + t * 16;
+  float* slot = red + team * Shape::RED + block * (Shape::VALUES * F3R_FEATURES * MP) + f;
+  unsigned long long* first_half = half_done + 2 * team + block;
+  bool ok = true, again = false;
+  unsigned turn = 0;                                             // parity of the team's items
+  // A team always meets the same stages: it has seen the phase before the one that it waits for, and a parity tells no more.
   // Past the end of K the copies bring zeros, which are multiplied like the rest: a branch around a chunk would keep the compiler from
   // working on two at a time (22,016 features x 2,048, one row: 32.5 -> 31.8 us; 2,048 x 11,008: 25.3 -> 19.2).
-  for (int i = s; i < items; i += S, parity ^= 1) {
-    float v[4][TILES][4];
+  for (int i = team; i < items; turn ^= 1, again = true) {
+    const int s = i % S;
     if (ok) {
-      ok = mbar_wait(full + s, parity);
+      ok = mbar_wait(full + s, (unsigned)(i / S) & 1);
       if (!ok && lane == 0) atomicExch(err, 53);
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-#pragma unroll
-      for (int n = 0; n < TILES; ++n) v[c][n][0] = v[c][n][1] = v[c][n][2] = v[c][n][3] = 0.f;
-      unsigned a[2][3][4], b[TILES][2][3][2];
+    float v[4][TILES][4];
+    unsigned a[2][2][3][4], b[2][TILES][2][3][2];
+    auto weights = [&](int c, unsigned (&parts)[2][3][4]) {      // of line c
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const unsigned at = wa + c * 128 + (((h * 4 + t) ^ ((f + half * 4 + c) & 7)) << 4);        // a block's 8 lines are a whole turn of the swizzle
+        const unsigned at = wa + s * Shape::STAGE + c * 128 + (((h * 4 + t) ^ ((f + line0 + c) & 7)) << 4);
         const ulonglong2 w0 = f3_lds(at), w1 = f3_lds(at + 8 * F3R_PITCH);
-        f3_split(w0.x, a[h][0][0], a[h][1][0], a[h][2][0]);
-        f3_split(w1.x, a[h][0][1], a[h][1][1], a[h][2][1]);
-        f3_split(w0.y, a[h][0][2], a[h][1][2], a[h][2][2]);
-        f3_split(w1.y, a[h][0][3], a[h][1][3], a[h][2][3]);
-#pragma unroll
-        for (int n = 0; n < TILES; ++n) {
-          const ulonglong2 x = f3_lds(xa + n * (8 * F3R_K * 4) + c * 128 + h * 64);
-          f3_split(x.x, b[n][h][0][0], b[n][h][1][0], b[n][h][2][0]);
-          f3_split(x.y, b[n][h][0][1], b[n][h][1][1], b[n][h][2][1]);
-        }
+        f3_split(w0.x, parts[h][0][0], parts[h][1][0], parts[h][2][0]);
+        f3_split(w1.x, parts[h][0][1], parts[h][1][1], parts[h][2][1]);
+        f3_split(w0.y, parts[h][0][2], parts[h][1][2], parts[h][2][2]);
+        f3_split(w1.y, parts[h][0][3], parts[h][1][3], parts[h][2][3]);
       }
-      constexpr int wp[6] = {2, 0, 1, 1, 0, 0}, xp[6] = {0, 2, 1, 0, 1, 0};
+    };
+    auto rows = [&](int c, unsigned (&parts)[TILES][2][3][2]) {
 #pragma unroll
-      for (int p = 0; p < 6; ++p)
+      for (int n = 0; n < TILES; ++n)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h) {
+          const ulonglong2 x = f3_lds(xa + s * Shape::STAGE + n * (8 * F3R_K * 4) + c * 128 + h * 64);
+          f3_split(x.x, parts[n][h][0][0], parts[n][h][1][0], parts[n][h][2][0]);
+          f3_split(x.y, parts[n][h][0][1], parts[n][h][1][1], parts[n][h][2][1]);
+        }
+    };
+    constexpr int wp[6] = {2, 0, 1, 1, 0, 0}, xp[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-          for (int n = 0; n < TILES; ++n) f3_mma(v[c][n], a[h][wp[p]], b[n][h][xp[p]]);
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int n = 0; n < TILES; ++n) v[c][n][0] = v[c][n][1] = v[c][n][2] = v[c][n][3] = 0.f;
+    if (MP < 8) {
+      // Two lines at a time, whose MMAs wait for one another in turn.  Column n of the MMA is row n mod MP of line n / MP of those that share.
+#pragma unroll
+      for (int c0 = 0; c0 < 4; c0 += 2) {
+        weights(c0, a[0]);
+        weights(c0 + 1, a[1]);
+        if (c0 == 0 || SHARE == 2) rows(c0, b[0]);
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) f3_mma(v[c0 + c][0], a[c][h][wp[p]], b[0][0][h][xp[p]]);
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        weights(c, a[0]);
+        rows(c, b[0]);
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int n = 0; n < TILES; ++n) f3_mma(v[c][n], a[0][h][wp[p]], b[0][n][h][xp[p]]);
+      }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(empty + s);
-    if (half == 0) {
-      if (i >= S && ok) {
-        ok = mbar_wait(red_empty + s, parity ^ 1);
+    if (MP < 8 || half == 0) {
+      if (again && ok) {
+        ok = mbar_wait(red_empty + team, turn ^ 1);
         if (!ok && lane == 0) atomicExch(err, 54);
       }
-      __syncwarp();
-    } else {
+    } else if (ok) {
       // within one phase: the first half comes again only behind red_empty, so behind this warp's red_full
-      if (ok) {
-        ok = mbar_wait(first_half, parity);
-        if (!ok && lane == 0) atomicExch(err, 59);
-      }
-      __syncwarp();
+      ok = mbar_wait(first_half, turn);
+      if (!ok && lane == 0) atomicExch(err, 59);
     }
+    __syncwarp();
 #pragma unroll
     for (int n = 0; n < TILES; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int m = n * 8 + 2 * t + (e & 1);
-        float* at = slot + m * F3R_FEATURES + 8 * (e >> 1);
-        if (m >= MP) continue;
-        float sum = half == 0 ? v[0][n][e] : *at + v[0][n][e];
-        sum += v[1][n][e];
-        sum += v[2][n][e];
-        *at = sum + v[3][n][e];
+        const int col = n * 8 + 2 * t + (e & 1);
+        float* at = slot + col % MP * F3R_FEATURES + 8 * (e >> 1);
+        if (MP < 8) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (col / MP == c % SHARE) at[(half * 4 + c) * (F3R_FEATURES * MP)] = v[c][n][e];
+        } else {
+          float sum = half == 0 ? v[0][n][e] : *at + v[0][n][e];
+          sum += v[1][n][e];
+          sum += v[2][n][e];
+          *at = sum + v[3][n][e];
+        }
       }
     __syncwarp();
-    if (lane == 0) mbar_arrive(half == 0 ? first_half : red_full + s);
+    if (lane == 0) mbar_arrive(MP >= 8 && half == 0 ? first_half : red_full + team);
+    i += s + TEAMS < S ? TEAMS : S - s + team;
   }
   }
   // every warp gets here: all waits are bounded
@@ -790,28 +847,34 @@ static bool f3_map_parts(CUtensorMap* map, void* base, int M, int K, int bn) {
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int MP>
+template <int MP, int TEAMS>
 static int f3_launch_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc,
-                          bool early, int* err, cudaStream_t s) {
-  using Shape = F3Rows<MP>;
+                          bool early, int* err, int sms, cudaStream_t s) {
+  using Shape = F3Rows<MP, TEAMS>;
   CUtensorMap mx, mw;
   if (!f3_map_lines(&mx, A, M, K, lda, MP, F3R_K / 32, false) || !f3_map_lines(&mw, W, N, K, ldw, F3R_FEATURES, 17, true)) return (int)cudaErrorInvalidValue;
-  const cudaError_t e = cudaFuncSetAttribute(f3_rows_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
+  const cudaError_t e = cudaFuncSetAttribute(f3_rows_kernel<MP, TEAMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
   if (e != cudaSuccess) return (int)e;
-  const int sms = device_sm_count(), groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
-  if (sms <= 0) return (int)cudaErrorInvalidDevice;
-  launch(f3_rows_kernel<MP>, dim3(groups < sms ? groups : sms), dim3(Shape::THREADS), Shape::SMEM, s, mx, mw, A, W, bias, C, M, N, K, lda, ldw,
+  const int groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
+  launch(f3_rows_kernel<MP, TEAMS>, dim3(groups < sms ? groups : sms), dim3(Shape::THREADS), Shape::SMEM, s, mx, mw, A, W, bias, C, M, N, K, lda, ldw,
          ldc, early, err);
   return launch_status();
 }
 
 int launch_f32x3_few(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc,
                      bool early, int* err, cudaStream_t s) {
-  if (M == 1) return f3_launch_rows<1>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
-  if (M == 2) return f3_launch_rows<2>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
-  if (M <= 4) return f3_launch_rows<4>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
-  if (M <= 8) return f3_launch_rows<8>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
-  return f3_launch_rows<16>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
+  const int sms = device_sm_count();
+  if (sms <= 0) return (int)cudaErrorInvalidDevice;
+  // Three teams leave their warps the registers for two lines at a time and end sooner; over a long stream of one row four ride over its
+  // unevenness (us with three and four: 2,048 x 11,008, 22 items a CTA, 17.4 and 18.0, 22,016 x 2,048, 40, 28.5 and 29.8; 3,584 x 18,944, 74,
+  // 59.8 and 54.5, 37,888 x 3,584, 112, 83.3 and 82.0, 151,936 x 2,048, 260, 188 and 177; two rows of the last two 79 and 90, 189 and 197).
+  const bool longer = (long long)((N + F3R_FEATURES - 1) / F3R_FEATURES + sms - 1) / sms * ((K + F3R_K - 1) / F3R_K) > 56;
+  if (M == 1 && longer) return f3_launch_rows<1, 4>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  if (M == 1) return f3_launch_rows<1, 3>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  if (M == 2) return f3_launch_rows<2, 3>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  if (M <= 4) return f3_launch_rows<4, 3>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  if (M <= 8) return f3_launch_rows<8, 4>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  return f3_launch_rows<16, 3>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
 }
 
 // How f3_tile_kernel takes a product: the width of its tiles, and into how many ranges of blocks a tile is cut.  The one that ends

@@ -18,7 +18,9 @@ def _product(a, w, b=None):
 #  rows, features, K, pitch of the rows beyond K: up to 16 rows a stream; more of them tiles of 32, 64, 96 and 128 rows, with K in parts (where the
 #  tiles are few) and whole
 CASES = [(1, 15, 256, 0), (2, 33, 288, 0), (3, 3000, 512, 4), (8, 2048, 544, 0), (9, 100, 1056, 0), (16, 16, 11008, 32),
-         (17, 127, 256, 0), (33, 129, 288, 0), (64, 2048, 2048, 0), (65, 7000, 320, 4), (97, 9472, 512, 0), (200, 9500, 800, 0), (300, 20000, 256, 12), (1000, 640, 4096, 0)]
+         (17, 127, 256, 0), (33, 129, 288, 0), (64, 2048, 2048, 0), (65, 7000, 320, 4), (97, 9472, 512, 0), (200, 9500, 800, 0), (300, 20000, 256, 12), (1000, 640, 4096, 0),
+         # up to four rows, whose lines share their parts: few features, K in one and several spans, a long stream
+         (5, 3, 512, 0), (5, 701, 6016, 4), (5, 33, 2080, 0), (17, 2500, 1280, 0), (5, 130, 18944, 0), (5, 9, 33024, 0), (5, 24000, 2560, 0)]
 
 
 @pytest.mark.parametrize("m,n,k,extra", CASES)
