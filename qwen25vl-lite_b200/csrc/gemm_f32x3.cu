@@ -164,7 +164,7 @@ __device__ __forceinline__ void f3_tma_3d_once(unsigned dst, const CUtensorMap* 
 }
 
 // ---- up to 16 rows: a stream of the weights -------------------------------------------------------------------------
-// One persistent CTA per SM; its items are (group of 16 features, 512 k), one stage of the ring each, which two copies fill: a
+// One persistent CTA per SM; its items are (group of 16 features, of small products with more rows also a group of 16 rows; 512 k), one stage of the ring each, which two copies fill: a
 // box of 16 rows of W and one of the rows of x (the copy engine takes a request about every 90 cycles whatever its size).  K is
 // seen as lines of 32; a row of W's box holds 17 of them, the last one not used, so that the 128-byte swizzle puts the same
 // line of eight rows into eight different bank groups.  A team of four warps has an item, half a block a warp: the weights are
@@ -179,8 +179,8 @@ __device__ __forceinline__ void f3_tma_3d_once(unsigned dst, const CUtensorMap* 
 // 27.4 / 28.4 / 28.8 / 30.6 / 44.5 (26.7 / 27.7 / 30.9 / 39.4 / 70.4), 2,048 x 11,008 16.2 / 17.6 / 17.8 / 18.5 / 26.5 (15.2 / 16.0 / 18.3 / 24.9 / 41),
 // 2,560 x 2,048 6.7 / 6.7 / 7.0 / 6.9 / 10.7 (5.0 / 5.5 / 6.5 / 8.6 / 15.8), 320 x 256 2.3 / 2.3 / 2.2 / 2.6 / 3.4 (2.2 / 2.2 / 2.5 / 3.4 / 3.6).
 // One and two rows stay behind FMA where the first stages arrive together: cutting up 32 KB takes four schedulers some 320 cycles, with every
-// team's 12 MMAs behind it.  Each line's rows cut up for itself, one line at a time, three quarters of an item's divisions by the number
-// of spans: 30.2, 18.7, 7.5 us for one row.  Two warps a stage: 35, 21; stages of 256 k: 39, 23; sixteen warps with a chunk each of every
+// team's 12 MMAs behind it.  With every line's rows cut up for itself, a line at a time, and divisions in the producer and the adding warp one
+// row took 30.2, 18.7 and 7.5 us.  Two warps a stage: 35, 21; stages of 256 k: 39, 23; sixteen warps with a chunk each of every
 // stage: 37, 22; two teams of eight warps with two lines each: 32, 20; lines as the MMA's rows and items of 4 features x 2,048 k, the rows
 // in shared memory whole: 28.3, 17.0, but 15.3 for 4,608 x 3,584 (12.4).
 #define F3R_FEATURES 16
@@ -221,8 +221,9 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   unsigned long long* half_done = red_empty + TEAMS;             // two of each team, one a block
   int* odd = reinterpret_cast<int*>(half_done + 2 * TEAMS);      // a result is not finite
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int spans = (K + F3R_K - 1) / F3R_K, groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
-  const int items = ((groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * spans;
+  // its items are the spans of units: a group of features of a group of MP rows
+  const int spans = (K + F3R_K - 1) / F3R_K, row_groups = (M + MP - 1) / MP, units = (N + F3R_FEATURES - 1) / F3R_FEATURES * row_groups;
+  const int items = ((units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * spans;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -246,16 +247,25 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     if (lane == 0) {
       const unsigned long long once = l2_evict_first();
       // counters: a division stands between a stage that is free and its copies
-      struct { int line, n0; } w = {0, (int)blockIdx.x * F3R_FEATURES}, x = {0, 0};
+      struct { int line, unit, at; } w = {0, (int)blockIdx.x, (int)blockIdx.x / row_groups * F3R_FEATURES}, x = {0, (int)blockIdx.x, (int)blockIdx.x % row_groups * MP};
       const int end = spans * (F3R_K / 32);
       auto weights = [&](int s) {
         mbar_expect_tx(full + s, Shape::STAGE);
-        f3_tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.n0, full + s, once);
-        if ((w.line += F3R_K / 32) == end) w = {0, w.n0 + (int)gridDim.x * F3R_FEATURES};
+        if (row_groups == 1) f3_tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.at, full + s, once);
+        else f3_tma_3d(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.at, full + s);                  // the next group of rows reads them too
+        if ((w.line += F3R_K / 32) == end) {
+          w.line = 0;
+          w.unit += (int)gridDim.x;
+          w.at = w.unit / row_groups * F3R_FEATURES;
+        }
       };
       auto rows = [&](int s) {
-        f3_tma_3d(smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES, &map_x, 0, x.line, 0, full + s);
-        if ((x.line += F3R_K / 32) == end) x.line = 0;
+        f3_tma_3d(smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES, &map_x, 0, x.line, x.at, full + s);
+        if ((x.line += F3R_K / 32) == end) {
+          x.line = 0;
+          x.unit += (int)gridDim.x;
+          x.at = x.unit % row_groups * MP;
+        }
       };
       const int ahead = min(S, items);
       if (!early) pdl_wait();
@@ -281,7 +291,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 #pragma unroll
     for (int v = 0; v < V; ++v) total[v] = 0.f;
     unsigned parities = 0;                                       // a bit for each team
-    int span = 0, g = (int)blockIdx.x;
+    int span = 0, unit = (int)blockIdx.x;
     for (int i = 0; i < items; ++i) {
       const int team = i % S % TEAMS;
       if (ok) {
@@ -305,10 +315,10 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(red_empty + team);
       if (++span == spans) {
-        const int n = g * F3R_FEATURES + (lane & 15);
+        const int n = unit / row_groups * F3R_FEATURES + (lane & 15), m0 = unit % row_groups * MP + (lane >> 4);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-          const int m = v * 2 + (lane >> 4);
+          const int m = m0 + v * 2;
           if (m < M && n < N && (MP > 1 || lane < F3R_FEATURES)) {
             const float value = total[v] + (bias ? bias[n] : 0.f);
             C[(size_t)m * ldc + n] = value;
@@ -317,7 +327,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           total[v] = 0.f;
         }
         span = 0;
-        g += (int)gridDim.x;
+        unit += (int)gridDim.x;
       }
     }
   } else {
@@ -434,8 +444,10 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   // every warp gets here: all waits are bounded
   __syncthreads();
   if (*odd != 0) {
-    for (int g = blockIdx.x; g < groups; g += gridDim.x)
-      f3_again(A, W, bias, C, reinterpret_cast<unsigned*>(smem), 0, M, g * F3R_FEATURES, min(N, (g + 1) * F3R_FEATURES), K, lda, ldw, ldc);
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+      const int n0 = unit / row_groups * F3R_FEATURES, m0 = unit % row_groups * MP;
+      f3_again(A, W, bias, C, reinterpret_cast<unsigned*>(smem), m0, min(MP, M - m0), n0, min(N, n0 + F3R_FEATURES), K, lda, ldw, ldc);
+    }
   }
 }
 
@@ -855,8 +867,8 @@ static int f3_launch_rows(const float* A, const float* W, const float* bias, flo
   if (!f3_map_lines(&mx, A, M, K, lda, MP, F3R_K / 32, false) || !f3_map_lines(&mw, W, N, K, ldw, F3R_FEATURES, 17, true)) return (int)cudaErrorInvalidValue;
   const cudaError_t e = cudaFuncSetAttribute(f3_rows_kernel<MP, TEAMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
   if (e != cudaSuccess) return (int)e;
-  const int groups = (N + F3R_FEATURES - 1) / F3R_FEATURES;
-  launch(f3_rows_kernel<MP, TEAMS>, dim3(groups < sms ? groups : sms), dim3(Shape::THREADS), Shape::SMEM, s, mx, mw, A, W, bias, C, M, N, K, lda, ldw,
+  const int units = (N + F3R_FEATURES - 1) / F3R_FEATURES * ((M + MP - 1) / MP);
+  launch(f3_rows_kernel<MP, TEAMS>, dim3(units < sms ? units : sms), dim3(Shape::THREADS), Shape::SMEM, s, mx, mw, A, W, bias, C, M, N, K, lda, ldw,
          ldc, early, err);
   return launch_status();
 }
@@ -879,19 +891,19 @@ int launch_f32x3_few(const float* A, const float* W, const float* bias, float* C
 
 // How f3_tile_kernel takes a product: the width of its tiles, and into how many ranges of blocks a tile is cut.  The one that ends
 // first: the chunks of the fullest SM at what a chunk takes (ns), and for a split the trip through its planes.
-struct F3Plan { int bn, splits; };
+struct F3Plan { int bn, splits; double ns; };
 static F3Plan f3_plan(int M, int N, int K, int sms) {
   const int widths[4] = {128, 96, 64, 32}, ns[4] = {640, 540, 455, 425};
   const int blocks = (K + F3_BLOCK - 1) / F3_BLOCK;
   const double planes = 4.0 * blocks * M * N;
-  F3Plan best = {128, 1};
+  F3Plan best = {128, 1, 0};
   double least = -1;
   for (int i = 0; i < 4; ++i) {
     const long long tiles = (long long)((M + widths[i] - 1) / widths[i]) * ((N + 127) / 128);
     const long long room = sms / tiles;
     const int splits = planes <= 64e6 ? (int)(room < 1 ? 1 : room < blocks ? room : blocks) : 1;
     double t = splits > 1 ? 8.0 * ((blocks + splits - 1) / splits) * ns[i] + 3000 + planes / 2000 : (double)((tiles + sms - 1) / sms) * (K / F3_CHUNK) * ns[i];
-    if (least < 0 || t < least) { best = {widths[i], splits}; least = t; }
+    if (least < 0 || t < least) { best = {widths[i], splits, t}; least = t; }
   }
   return best;
 }
@@ -920,10 +932,17 @@ int launch_f32x3_many(const float* A, const float* W, const float* bias, float* 
                       bool early, int* err, cudaStream_t s) {
   const int sms = device_sm_count();
   if (sms <= 0) return (int)cudaErrorInvalidDevice;
+  const F3Plan plan = f3_plan(M, N, K, sms);
+  // Small products, as groups of 16 rows: one launch instead of two or three.  An item takes 1.1 us and the launch 2.5; tiles have 2.4 us of
+  // launches around them, a split one 2 more than its plan counts (us by tiles and this way: 17 rows x 320 features x 256 6.2 and 3.7, 64 x 320 x 512
+  // 7.5 and 3.6, 64 x 1,024 x 512 8.0 and 5.5, 17 x 1,024 x 1,024 7.6 and 5.3; 64 x 4,096 x 512 stays with the tiles at 9.5).
+  const long long units = (long long)((N + F3R_FEATURES - 1) / F3R_FEATURES) * ((M + 15) / 16);
+  if (lda % 4 == 0 && lda >= K && !((uintptr_t)A & 15) && units < 1 << 16 &&
+      1100.0 * ((units + sms - 1) / sms) * ((K + F3R_K - 1) / F3R_K) + 2500 < plan.ns + (plan.splits > 1 ? 2000 : 2400))
+    return f3_launch_rows<16, 3>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
   const size_t most = (size_t)sms * 8, eighths = ((size_t)M * (K / 8) + 255) / 256, elements = ((size_t)M * N + 255) / 256;
   launch(f3_parts_kernel, dim3((unsigned)(eighths < most ? eighths : most)), dim3(256), 0, s, A, (uint4*)scratch, M, K, lda,
          lda % 4 == 0 && !((uintptr_t)A & 15));
-  const F3Plan plan = f3_plan(M, N, K, sms);
   float* planes = reinterpret_cast<float*>(static_cast<char*>(scratch) + f3_parts_bytes(M, K));
   int e;
   if (plan.bn == 128) e = f3_launch_tiles<128>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);

@@ -20,7 +20,9 @@ def _product(a, w, b=None):
 CASES = [(1, 15, 256, 0), (2, 33, 288, 0), (3, 3000, 512, 4), (8, 2048, 544, 0), (9, 100, 1056, 0), (16, 16, 11008, 32),
          (17, 127, 256, 0), (33, 129, 288, 0), (64, 2048, 2048, 0), (65, 7000, 320, 4), (97, 9472, 512, 0), (200, 9500, 800, 0), (300, 20000, 256, 12), (1000, 640, 4096, 0),
          # up to four rows, whose lines share their parts: few features, K in one and several spans, a long stream
-         (5, 3, 512, 0), (5, 701, 6016, 4), (5, 33, 2080, 0), (17, 2500, 1280, 0), (5, 130, 18944, 0), (5, 9, 33024, 0), (5, 24000, 2560, 0)]
+         (5, 3, 512, 0), (5, 701, 6016, 4), (5, 33, 2080, 0), (17, 2500, 1280, 0), (5, 130, 18944, 0), (5, 9, 33024, 0), (5, 24000, 3072, 0),
+         # more than 16 rows: small products as groups of 16 rows, larger ones as tiles of each width
+         (50, 300, 1056, 0), (130, 129, 512, 8), (17, 5000, 256, 0), (40, 9000, 288, 0), (90, 20000, 256, 0)]
 
 
 @pytest.mark.parametrize("m,n,k,extra", CASES)
@@ -47,7 +49,7 @@ def test_rows_that_are_not_aligned(m):
         assert torch.equal(_product(a, w), _product(a.clone(), w))
 
 
-@pytest.mark.parametrize("m,n", [(3, 260), (16, 260), (40, 260), (300, 260), (300, 9600)])
+@pytest.mark.parametrize("m,n", [(3, 260), (16, 260), (40, 260), (40, 9600), (300, 260), (300, 9600)])
 def test_operands_without_three_parts(m, n):
     gen = torch.Generator(device="cuda").manual_seed(m)
     a, w = torch.randn(m, 512, generator=gen, device="cuda"), torch.randn(n, 512, generator=gen, device="cuda")
