@@ -801,8 +801,8 @@ f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, con
     const float more = bias ? bias[n] : 0.f;
     total += more;
     for (unsigned todo = __ballot_sync(0xffffffffu, !f3_finite(total)); todo != 0; todo &= todo - 1) {
-      const int from = __ffs(todo) - 1;
-      const float* a = A + (size_t)__shfl_sync(0xffffffffu, m, from) * lda;
+      const int from = __ffs(todo) - 1, row = __shfl_sync(0xffffffffu, m, from);
+      const float* a = A + (size_t)row * lda;
       const float* w = W + (size_t)__shfl_sync(0xffffffffu, n, from) * ldw;
       float sum = 0.f;                           // as f3_plain has it
       bool nan = false;                          // the row holds one: nothing else can come of it
@@ -816,6 +816,7 @@ f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, con
         }
         nan = __any_sync(0xffffffffu, nan);
       }
+      if (nan) todo &= ~__ballot_sync(0xffffffffu, m == row) | 1u << from;
       sum = warp_sum(sum) + more;
       if (lane == from && !nan) total = sum;
     }
