@@ -572,6 +572,8 @@ static int launch_tile(const float* A, const float* W, const float* bias, float*
 // aligned, for products that the tensor cores take, but not for up to F32X3_FEW rows that are aligned to 16 bytes.  err: device int that
 // gets a code if a bounded wait gave up.
 Q25_EXPORT long long q25_gemm_f32_scratch(int M, int N, int K) { return M > 0 && N > 0 && f32x3_takes(K) ? (long long)f32x3_scratch(M, N, K) : 0; }
+// Kernels that this thread's last product on tensor cores with scratch memory was.
+Q25_EXPORT int q25_gemm_f32_launches() { return f32x3_launches; }
 Q25_EXPORT int q25_gemm_f32(const float* A, const float* W, const float* bias, float* C, void* scratch, int M, int N, int K, int lda,
                             int ldw, int ldc, int fixed, int* err, void* stream) {
   if (M <= 0 || N <= 0) return 0;

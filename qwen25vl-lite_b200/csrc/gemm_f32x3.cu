@@ -929,6 +929,7 @@ static int f3_launch_tiles(const float* A, const float* W, const float* bias, fl
   return launch_status();
 }
 
+thread_local int f32x3_launches = 1;             // of this thread's last product of more than F32X3_FEW rows
 int launch_f32x3_many(const float* A, const float* W, const float* bias, float* C, void* scratch, int M, int N, int K, int lda, int ldw, int ldc,
                       bool early, int* err, cudaStream_t s) {
   const int sms = device_sm_count();
@@ -939,8 +940,10 @@ int launch_f32x3_many(const float* A, const float* W, const float* bias, float* 
   // 7.5 and 3.6, 64 x 1,024 x 512 8.0 and 5.5, 17 x 1,024 x 1,024 7.6 and 5.3; 64 x 4,096 x 512 stays with the tiles at 9.5).
   const long long units = (long long)((N + F3R_FEATURES - 1) / F3R_FEATURES) * ((M + 15) / 16);
   if (lda % 4 == 0 && lda >= K && !((uintptr_t)A & 15) && units < 1 << 16 &&
-      1100.0 * ((units + sms - 1) / sms) * ((K + F3R_K - 1) / F3R_K) + 2500 < plan.ns + (plan.splits > 1 ? 2000 : 2400))
+      1100.0 * ((units + sms - 1) / sms) * ((K + F3R_K - 1) / F3R_K) + 2500 < plan.ns + (plan.splits > 1 ? 2000 : 2400)) {
+    f32x3_launches = 1;
     return f3_launch_rows<16, 3>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  }
   const size_t most = (size_t)sms * 8, eighths = ((size_t)M * (K / 8) + 255) / 256, elements = ((size_t)M * N + 255) / 256;
   launch(f3_parts_kernel, dim3((unsigned)(eighths < most ? eighths : most)), dim3(256), 0, s, A, (uint4*)scratch, M, K, lda,
          lda % 4 == 0 && !((uintptr_t)A & 15));
@@ -950,6 +953,7 @@ int launch_f32x3_many(const float* A, const float* W, const float* bias, float* 
   else if (plan.bn == 96) e = f3_launch_tiles<96>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);
   else if (plan.bn == 64) e = f3_launch_tiles<64>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);
   else e = f3_launch_tiles<32>(A, W, bias, C, scratch, planes, plan.splits, M, N, K, lda, ldw, ldc, early, err, sms, s);
+  f32x3_launches = plan.splits == 1 ? 2 : 3;
   if (e != 0 || plan.splits == 1) return e;
   launch(f3_sum_kernel, dim3((unsigned)(elements < most ? elements : most)), dim3(256), 0, s, planes, A, W, bias, C, M, N, K, lda, ldw, ldc);
   return launch_status();

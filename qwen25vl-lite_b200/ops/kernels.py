@@ -484,7 +484,8 @@ F32X3_SCRATCH = 1 << 28       # bytes that the parts of a product's rows may tak
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, fixed: bool = False) -> None:
     """out[M,N] = a[M,K] . w[N,K]^T + bias in true 32 bits: by FMA, or from K 256 on (multiples of 32) on tensor cores with every number
-    cut into three exact parts.  A row's bits depend on nothing but K.  ``fixed``: ``w`` is a weight that no kernel writes, and is
+    cut into three exact parts.  A row's bits depend on nothing but K, and on whether ``w``'s rows are aligned to 16 bytes (from K 256 on
+    others stay with FMA).  ``fixed``: ``w`` is a weight that no kernel writes, and is
     fetched before the kernel ahead on the stream has ended."""
     m, k = a.shape
     n = w.shape[0]
@@ -495,7 +496,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
             raise KernelError(f"gemm_f32 {what}: needs a float32 CUDA matrix with unit inner stride")
     lda = a.stride(0) if m > 1 else k
     scratch = None            # the three bfloat16 parts of a's values, and sums of parts of K, where the tensor cores take more than a few rows
-    if k >= 256 and k % 32 == 0 and (m > F32X3_FEW or lda % 4 or lda < k or a.data_ptr() % 16):
+    tensor_cores = k >= 256 and k % 32 == 0 and w.data_ptr() % 16 == 0 and (n == 1 or w.stride(0) % 4 == 0 and w.stride(0) >= k)
+    if tensor_cores and (m > F32X3_FEW or lda % 4 or lda < k or a.data_ptr() % 16):
         slab = max(384, F32X3_SCRATCH // (6 * k) // 384 * 384)              # whole tiles of 128 and of 96 rows
         if m > slab:
             for at in range(0, m, slab):
@@ -507,6 +509,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     _check(_fn("q25_gemm_f32", _UNTYPED["q25_gemm_f32"])(
         a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _ptr(scratch), m, n, k, lda, w.stride(0), out.stride(0),
         int(fixed), error_flag(out.device).data_ptr(), _stream()), "gemm_f32")
+    if scratch is not None:
+        count_replayed(_fn("q25_gemm_f32_launches", [])() - 1)              # up to three kernels by one call
 
 
 SKINNY_STORE, SKINNY_BIAS, SKINNY_F32, SKINNY_SWIGLU, SKINNY_RESIDUAL, SKINNY_GLU, SKINNY_RELU2, SKINNY_RESIDUAL_SCALED = 0, 1, 2, 3, 4, 5, 6, 7

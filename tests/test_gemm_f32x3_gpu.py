@@ -105,3 +105,29 @@ def test_rows_that_are_not_numbers(m, n, k):
     assert torch.equal(out[m // 2], w[:, k - 1].sign() * float("inf"))
     rest = [i for i in range(m) if i != m // 2]
     assert torch.equal(out[rest], whole[rest])
+
+
+@pytest.mark.parametrize("m,n,k,kernels_of_it", [(16, 300, 512, 1), (40, 300, 512, 1), (300, 20000, 256, 2), (64, 2048, 2048, 3)])
+def test_launches_are_counted(m, n, k, kernels_of_it):
+    from qwen25vl_lite.ops import kernels
+    a, w = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda")
+    _product(a, w)
+    before = kernels.launch_count()
+    kernels.gemm_f32(a, w, None, torch.empty(m, n, device="cuda"))
+    assert kernels.launch_count() - before == kernels_of_it
+
+
+def test_a_second_operand_that_is_not_aligned_takes_no_scratch_memory():
+    """It stays with the FMA kernels (in their order), whatever the number of rows."""
+    from qwen25vl_lite.ops import kernels
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a, flat = torch.randn(3000, 512, generator=gen, device="cuda"), torch.randn(64 * 512 + 1, generator=gen, device="cuda")
+    w, out = flat[1:].view(64, 512), torch.empty(3000, 64, device="cuda")
+    kernels.gemm_f32(a, w, None, out)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before, launched = torch.cuda.memory_allocated(), kernels.launch_count()
+    kernels.gemm_f32(a, w, None, out)
+    assert torch.cuda.max_memory_allocated() == before and kernels.launch_count() - launched == 1
+    want = a.double() @ w.double().T
+    assert float((out.double() - want).norm() / want.norm()) < 3e-7
