@@ -2,7 +2,7 @@
 //
 // A 32-bit number is the sum of three bfloat16 numbers, hi + mid + lo: hi is the number rounded, mid what hi leaves, rounded,
 // lo the rest; 8 bits of the mantissa each, so nothing is lost (below 2^-109 the rest is less than bfloat16's smallest number, and low
-// bits are lost: of a sum in which such operands alone count, 2e-6 at 2^-116).  Of the nine products of two such sums the six largest are taken;
+// bits are lost; results so small that this could be seen are computed again).  Of the nine products of two such sums the six largest are taken;
 // the others (mid lo, lo mid, lo lo) are below 2^-24 of the product.  bfloat16 products are exact in 32 bits, what remains is how
 // they are added.  The tensor core cuts bits off where FMA rounds, so it adds no more than 32 k (two instructions of 16 k for
 // each of the six, the small ones first); the values of these chunks are added by ordinary 32-bit additions.  For every
@@ -18,8 +18,8 @@
 // Error against 64 bits, relative 2-norm, random operands of both signs, by FMA (gemm_f32.cu) and here: K 256 1.49e-7 and 8.0e-8, 2,048
 // 1.66e-7 and 9.8e-8, 11,008 2.24e-7 and 1.46e-7.  Sums of one sign collect what is cut off: 6.0e-8 and 7.1e-8 at K 512, 7.0e-8 and
 // 7.3e-8 at 2,048, 1.33e-7 and 1.08e-7 at 11,008.
-// A result that is not finite (an infinite or not-a-number operand has no three parts; a part may round up to infinity) is
-// computed again by plain FMA, behind its CTA's pipeline.
+// A result that is not finite (an infinite or not-a-number operand has no three parts; a part may round up to infinity), or below 2^-84
+// and not zero, is computed again by plain FMA, behind its CTA's pipeline.
 //
 //   * up to 16 rows (decode steps): f3_rows_kernel, a stream of the weights, mma.sync;
 //   * more rows: f3_parts_kernel cuts A into its three parts, f3_tile_kernel multiplies, tcgen05; where its tiles are too few
@@ -61,9 +61,14 @@ __device__ __forceinline__ ulonglong2 f3_lds(unsigned addr) {
   asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];\n" : "=l"(v.x), "=l"(v.y) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ bool f3_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+// Neither infinite nor not a number, nor so small that what operands lose below 2^-109 would be seen: at most 2^-134 each, times partners
+// up to 2^10, 2^15 of them, is below half a unit in the last place of 2^-84.
+__device__ __forceinline__ bool f3_sound(float v) {
+  const float size = fabsf(v);
+  return size <= 3.402823466e38f && (size >= 0x1p-84f || size == 0.f);
+}
 
-// ---- results that are not finite --------------------------------------------------------------------------------------
+// ---- results that are not finite, or very small --------------------------------------------------------------------------------------
 // They are marked where they are stored and computed again when their CTA's pipeline has ended: a dot product of 11,008 terms takes
 // some microseconds, during which warps with bounded waits would stand.
 //
@@ -118,7 +123,7 @@ __device__ __noinline__ void f3_again(const float* __restrict__ A, const float* 
     bool looked = false, nan = false;
     for (int i = 0; i < words; ++i) {
       const int n = n0 + i * 32 + lane;
-      unsigned mark = nan ? 0 : __ballot_sync(0xffffffffu, n < n1 && !f3_finite(__ldcg(C + (size_t)(m0 + r) * ldc + min(n, n1 - 1))));
+      unsigned mark = nan ? 0 : __ballot_sync(0xffffffffu, n < n1 && !f3_sound(__ldcg(C + (size_t)(m0 + r) * ldc + min(n, n1 - 1))));
       for (int k = lane; mark != 0 && !looked && !nan && k < K; k += 128) {      // K is a multiple of 32: the lanes go together
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -219,7 +224,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   unsigned long long* red_full = empty + S;
   unsigned long long* red_empty = red_full + TEAMS;
   unsigned long long* half_done = red_empty + TEAMS;             // two of each team, one a block
-  int* odd = reinterpret_cast<int*>(half_done + 2 * TEAMS);      // a result is not finite
+  int* odd = reinterpret_cast<int*>(half_done + 2 * TEAMS);      // a result is not sound
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // its items are the spans of units: a group of features of a group of MP rows
   const int spans = (K + F3R_K - 1) / F3R_K, row_groups = (M + MP - 1) / MP, units = (N + F3R_FEATURES - 1) / F3R_FEATURES * row_groups;
@@ -322,7 +327,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
           if (m < M && n < N && (MP > 1 || lane < F3R_FEATURES)) {
             const float value = total[v] + (bias ? bias[n] : 0.f);
             C[(size_t)m * ldc + n] = value;
-            if (!f3_finite(value)) *odd = 1;
+            if (!f3_sound(value)) *odd = 1;
           }
           total[v] = 0.f;
         }
@@ -563,7 +568,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
   // of each of the two buffers (a stage of W's parts and an accumulator): both are free for the MMAs; these have ended
   unsigned long long *ready = x_empty + XS, *done = ready + 2;
   unsigned* tmem_at = reinterpret_cast<unsigned*>(done + 2);
-  int* odd = reinterpret_cast<int*>(tmem_at + 1);                // a result is not finite
+  int* odd = reinterpret_cast<int*>(tmem_at + 1);                // a result is not sound
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int W_WARP = Shape::DRAINS + 4 * SETS, X_WARP = W_WARP + 1, MMA_WARP = W_WARP + 2;
   const int row_tiles = (M + BN - 1) / BN, tiles = row_tiles * ((N + 127) / 128);
@@ -750,7 +755,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 #pragma unroll
           for (int j = 0; j < WIDTH; ++j, dst += pitch) {
             const float value = acc[j] + more;
-            finite &= f3_finite(value);
+            finite &= f3_sound(value);
             if (m0 + j < M) *dst = value;
             asm volatile("" : "+l"(dst));        // one address after the other: all of them at once do not fit the registers
           }
@@ -800,7 +805,7 @@ f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, con
     }
     const float more = bias ? bias[n] : 0.f;
     total += more;
-    for (unsigned todo = __ballot_sync(0xffffffffu, !f3_finite(total)); todo != 0; todo &= todo - 1) {
+    for (unsigned todo = __ballot_sync(0xffffffffu, !f3_sound(total)); todo != 0; todo &= todo - 1) {
       const int from = __ffs(todo) - 1, row = __shfl_sync(0xffffffffu, m, from);
       const float* a = A + (size_t)row * lda;
       const float* w = W + (size_t)__shfl_sync(0xffffffffu, n, from) * ldw;
