@@ -1,4 +1,5 @@
-// Two floats in one 64-bit register pair, and the packed FMA on them: what the 32-bit kernels (gemm_f32.cu, attention_f32.cu) share.
+// Two floats in one 64-bit register pair, and the packed FMA on them: what the 32-bit kernels (gemm_f32.cu, gemm_f32x3.cu,
+// attention_f32.cu) share.
 #pragma once
 
 typedef unsigned long long f32x2;                // the lower one in the low word
@@ -21,4 +22,10 @@ __device__ __forceinline__ float2 split2(f32x2 v) {
 __device__ __forceinline__ float sum2(f32x2 v) {
   const float2 r = split2(v);
   return r.x + r.y;
+}
+// Two such pairs out of shared memory.
+__device__ __forceinline__ ulonglong2 lds_pair(unsigned addr) {
+  ulonglong2 v;
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];\n" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+  return v;
 }

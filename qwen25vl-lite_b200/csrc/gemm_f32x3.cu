@@ -56,11 +56,6 @@ __device__ __forceinline__ void f3_split(f32x2 x, unsigned& hi, unsigned& mid, u
   lo = f3_pack(v.x, v.y);
 }
 
-__device__ __forceinline__ ulonglong2 f3_lds(unsigned addr) {
-  ulonglong2 v;
-  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];\n" : "=l"(v.x), "=l"(v.y) : "r"(addr));
-  return v;
-}
 // Neither infinite nor not a number, nor so small that what operands lose below 2^-109 would be seen: at most 2^-134 each, times partners
 // up to 2^10, 2^15 of them, is below half a unit in the last place of 2^-84.
 __device__ __forceinline__ bool f3_sound(float v) {
@@ -154,20 +149,6 @@ __device__ __noinline__ void f3_again(const float* __restrict__ A, const float* 
   __syncthreads();                                               // the marks are free
 }
 
-__device__ __forceinline__ void f3_tma_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
-               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void f3_tma_3d(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
-               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
-}
-__device__ __forceinline__ void f3_tma_3d_once(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar,
-                                               unsigned long long policy) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;\n"
-               ::"r"(dst), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "l"(policy) : "memory");
-}
-
 // ---- up to 16 rows: a stream of the weights -------------------------------------------------------------------------
 // One persistent CTA per SM; its items are (group of 16 features, of small products with more rows also a group of 16 rows; 512 k), one stage of the ring each, which two copies fill: a
 // box of 16 rows of W and one of the rows of x (the copy engine takes a request about every 90 cycles whatever its size).  K is
@@ -256,8 +237,8 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       const int end = spans * (F3R_K / 32);
       auto weights = [&](int s) {
         mbar_expect_tx(full + s, Shape::STAGE);
-        if (row_groups == 1) f3_tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.at, full + s, once);
-        else f3_tma_3d(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.at, full + s);                  // the next group of rows reads them too
+        if (row_groups == 1) tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.at, full + s, once);
+        else tma_3d(smem_u32(smem + s * Shape::STAGE), &map_w, 0, w.line, w.at, full + s);                  // the next group of rows reads them too
         if ((w.line += F3R_K / 32) == end) {
           w.line = 0;
           w.unit += (int)gridDim.x;
@@ -265,7 +246,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         }
       };
       auto rows = [&](int s) {
-        f3_tma_3d(smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES, &map_x, 0, x.line, x.at, full + s);
+        tma_3d(smem_u32(smem + s * Shape::STAGE) + F3R_W_BYTES, &map_x, 0, x.line, x.at, full + s);
         if ((x.line += F3R_K / 32) == end) {
           x.line = 0;
           x.unit += (int)gridDim.x;
@@ -362,7 +343,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const unsigned at = wa + s * Shape::STAGE + c * 128 + (((h * 4 + t) ^ ((f + line0 + c) & 7)) << 4);
-        const ulonglong2 w0 = f3_lds(at), w1 = f3_lds(at + 8 * F3R_PITCH);
+        const ulonglong2 w0 = lds_pair(at), w1 = lds_pair(at + 8 * F3R_PITCH);
         f3_split(w0.x, parts[h][0][0], parts[h][1][0], parts[h][2][0]);
         f3_split(w1.x, parts[h][0][1], parts[h][1][1], parts[h][2][1]);
         f3_split(w0.y, parts[h][0][2], parts[h][1][2], parts[h][2][2]);
@@ -374,7 +355,7 @@ f3_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       for (int n = 0; n < TILES; ++n)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const ulonglong2 x = f3_lds(xa + s * Shape::STAGE + n * (8 * F3R_K * 4) + c * 128 + h * 64);
+          const ulonglong2 x = lds_pair(xa + s * Shape::STAGE + n * (8 * F3R_K * 4) + c * 128 + h * 64);
           f3_split(x.x, parts[n][h][0][0], parts[n][h][1][0], parts[n][h][2][0]);
           f3_split(x.y, parts[n][h][0][1], parts[n][h][1][1], parts[n][h][2][1]);
         }
@@ -594,7 +575,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
   auto load_w = [&](int it) {
     const int tile = first_tile + it / chunks * step, s = it % WS;
     mbar_expect_tx(w_full + s, Shape::WSTAGE);
-    f3_tma_2d(smem_u32(wring + s * Shape::WSTAGE), &map_w, (c_begin + it % chunks) * F3_CHUNK, tile / row_tiles * 128, w_full + s);
+    tma_2d(smem_u32(wring + s * Shape::WSTAGE), &map_w, (c_begin + it % chunks) * F3_CHUNK, tile / row_tiles * 128, w_full + s);
   };
   const int ahead = min(WS, mine);
   if (early && warp == W_WARP && lane == 0)
@@ -634,7 +615,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             if (!ok) { atomicExch(err, 56); break; }
           }
           mbar_expect_tx(x_full + s, Shape::XSTAGE);
-          f3_tma_3d(smem_u32(xring + s * Shape::XSTAGE), &map_p, c * F3_CHUNK, tile % row_tiles * BN, 0, x_full + s);
+          tma_3d(smem_u32(xring + s * Shape::XSTAGE), &map_p, c * F3_CHUNK, tile % row_tiles * BN, 0, x_full + s);
         }
       mbar_landed(x_full, XS, xt);
     }
@@ -684,7 +665,7 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
       const unsigned at = smem_u32(wring + s * Shape::WSTAGE) + row * 128;
       ulonglong2 v[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) v[c] = f3_lds(at + ((c ^ (row & 7)) << 4));
+      for (int c = 0; c < 8; ++c) v[c] = lds_pair(at + ((c ^ (row & 7)) << 4));
       unsigned p[3][16];
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
@@ -830,29 +811,6 @@ f3_sum_kernel(const float* __restrict__ planes, const float* __restrict__ A, con
 }
 
 // ---- host -----------------------------------------------------------------------------------------------------------
-// A [rows, K] float matrix of row pitch ld as lines of 32 k: boxes of box_rows x box_lines lines.
-static bool f3_map_lines(CUtensorMap* map, const float* base, int rows, int K, int ld, int box_rows, int box_lines, bool swizzle) {
-  EncodeTiledFn enc = encode_tiled();
-  if (!enc) return false;
-  const cuuint64_t dims[3] = {32, (cuuint64_t)(K / 32), (cuuint64_t)rows};
-  const cuuint64_t strides[2] = {128, (cuuint64_t)ld * 4};
-  const cuuint32_t box[3] = {32, (cuuint32_t)box_lines, (cuuint32_t)box_rows};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-// Boxes of 128 rows x 32 k of W.
-static bool f3_map_w(CUtensorMap* map, const float* base, int rows, int K, int ld) {
-  EncodeTiledFn enc = encode_tiled();
-  if (!enc) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  const cuuint32_t box[2] = {32, 128};
-  const cuuint32_t estr[2] = {1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 // Boxes of the three parts of bn rows x 64 k of A.
 static bool f3_map_parts(CUtensorMap* map, void* base, int M, int K, int bn) {
   EncodeTiledFn enc = encode_tiled();
@@ -870,7 +828,7 @@ static int f3_launch_rows(const float* A, const float* W, const float* bias, flo
                           bool early, int* err, int sms, cudaStream_t s) {
   using Shape = F3Rows<MP, TEAMS>;
   CUtensorMap mx, mw;
-  if (!f3_map_lines(&mx, A, M, K, lda, MP, F3R_K / 32, false) || !f3_map_lines(&mw, W, N, K, ldw, F3R_FEATURES, 17, true)) return (int)cudaErrorInvalidValue;
+  if (!make_blocks_f32(&mx, A, M, K, lda, MP, F3R_K / 32, false) || !make_blocks_f32(&mw, W, N, K, ldw, F3R_FEATURES, 17, true)) return (int)cudaErrorInvalidValue;
   const cudaError_t e = cudaFuncSetAttribute(f3_rows_kernel<MP, TEAMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
   if (e != cudaSuccess) return (int)e;
   const int units = (N + F3R_FEATURES - 1) / F3R_FEATURES * ((M + MP - 1) / MP);
@@ -925,7 +883,7 @@ static int f3_launch_tiles(const float* A, const float* W, const float* bias, fl
                            int K, int lda, int ldw, int ldc, bool early, int* err, int sms, cudaStream_t s) {
   using Shape = F3Tile<BN>;
   CUtensorMap mp, mw;
-  if (!f3_map_parts(&mp, parts, M, K, BN) || !f3_map_w(&mw, W, N, K, ldw)) return (int)cudaErrorInvalidValue;
+  if (!f3_map_parts(&mp, parts, M, K, BN) || !make_map_f32(&mw, W, N, K, ldw, 128)) return (int)cudaErrorInvalidValue;
   const cudaError_t e = cudaFuncSetAttribute(f3_tile_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
   if (e != cudaSuccess) return (int)e;
   const long long tiles = (long long)((M + BN - 1) / BN) * ((N + 127) / 128);
