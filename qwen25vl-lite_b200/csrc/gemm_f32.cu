@@ -1,8 +1,9 @@
 // C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) in true 32-bit.  This is the matrix product of the 32-bit path
 // (the reference's tested path is float32 end to end, src/qwen25vl_lite/engine.py:63).  Where K is 256 or more and a multiple of
-// 32 it runs on tensor cores, every number in three exact parts (gemm_f32x3.cu); this file has the others, plain FMA on the
-// CUDA cores.  (Figures below of longer K are from when these kernels took it.  The line lies at 256 because a row of 320 features
-// takes 2.0 us here and 3.3 there, where the start of a product counts for more; from 17 rows on 5.4 and 7.1.)
+// 32, and W's rows are aligned to 16 bytes, it runs on tensor cores, every number in three exact parts (gemm_f32x3.cu); this file has the
+// others, plain FMA on the CUDA cores.  (Figures of longer K below are from when these kernels took it.  The line lies at 256 because there the
+// two are even for one row and tensor cores ahead for more: 1 / 8 / 16 / 17 / 1,024 rows of 320 features, K 256, by FMA 2.2 / 3.4 / 3.6 / 5.4 / 11.5 us, there
+// 2.3 / 2.5 / 3.3 / 3.3 / 7.6; of 4,096 features 2.7 / 4.1 / 4.4 / 5.7 / 52 and 3.6 / 4.1 / 4.6 / 6.2 / 17.)
 //
 // Every output element is summed in one order, which all kernels of this file share: K is cut into
 // segments of 128; inside a segment the even and the odd k are one chain of fma each, in order,
@@ -91,25 +92,24 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 }
 
 // ---- up to 16 rows: a stream of the weights -------------------------------------------------------------------------
-// One persistent CTA per SM; its items are (group of 16 features, chunk of 512 k), one stage of the ring each, which two
-// copies fill: a box of 16 rows of W and one of the rows of x.  (The copy engine takes a request about every 90 cycles whatever
-// its size: as 16 boxes of 2 KB and four of x the stream ran at 5.2 TB/s.  22,016 features x 2,048 take 27 us for up to
-// two rows, 6.7 TB/s, 31 for four, 40 for eight and 71 for sixteen, where the reads of x out of shared memory count.)  K is seen as blocks of 32, and a row of W's box
-// holds 17 of them, the last one not used: with an odd number of 128-byte blocks a row, the 128-byte swizzle puts the
-// same block of eight rows into eight different bank groups.  A warp takes the items of one stage: lane = (pair of features p
-// and p + 8, segment of the chunk), so that 16 bytes of x serve two features, and leaves the segments' values in shared memory,
-// where the last warp adds them in order.  The producer starts the weights before it waits for the kernel before (early).
-// MT: rows of a lane; MG: warps that share a stage (rows 0 .. MT - 1 and MT ..).
+// One persistent CTA per SM; its items are groups of 16 features over all of K (below 256, as longer K runs in gemm_f32x3.cu), one stage of the
+// ring each, which two copies fill: a box of 16 rows of W and one of the rows of x.  (The copy engine takes a request about every
+// 90 cycles whatever its size.)  K is seen as blocks of 32, and a row of W's box holds 9 of them, the last one not used: with an odd number of
+// 128-byte blocks a row, the 128-byte swizzle puts the same block of eight rows into eight different bank groups.  A warp takes the
+// items of one stage: lane = (pair of features p and p + 8, segment), so that 16 bytes of x serve two features (the lanes beyond the two
+// segments of K idle), and leaves the segments' values in shared memory, where the last warp adds them in order.  The producer
+// starts the weights before it waits for the kernel before (early).  MT: rows of a lane; MG: warps that share a stage (rows 0 .. MT - 1
+// and MT ..).
 #define GR_ROWS 16
-#define GR_CHUNK 512
-#define GR_PITCH (17 * 128)                      // bytes between the rows of W in a stage
+#define GR_K 256                                 // k of a stage
+#define GR_PITCH (9 * 128)                       // bytes between the rows of W in a stage
 #define GR_W_BYTES (GR_ROWS * GR_PITCH)
 
 template <int MT, int MG> struct RowsShape {
   static constexpr int MP = MT * MG;
-  static constexpr int STAGE = GR_W_BYTES + MP * GR_CHUNK * 4;
+  static constexpr int STAGE = GR_W_BYTES + MP * GR_K * 4;
   static constexpr int STAGES = MP <= 4 ? 5 : MP == 8 ? 4 : 3;
-  static constexpr int RED = 4 * GR_ROWS * MP;                  // floats of one slot of segment values
+  static constexpr int RED = GR_K / GF_SEG * GR_ROWS * MP;      // floats of one slot of segment values
   static constexpr int WARPS = STAGES * MG;
   static constexpr int THREADS = (WARPS + 2) * 32;
   static constexpr int SMEM = 1024 + STAGES * (STAGE + RED * 4) + STAGES * 4 * 8;
@@ -129,8 +129,7 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   unsigned long long* red_full = empty + S;
   unsigned long long* red_empty = red_full + S;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int chunks = (K + GR_CHUNK - 1) / GR_CHUNK, groups = (N + GR_ROWS - 1) / GR_ROWS;
-  const int items = ((groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * chunks;
+  const int groups = (N + GR_ROWS - 1) / GR_ROWS, items = (groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -150,13 +149,13 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       const unsigned long long once = l2_evict_first();
       bool ok = true;
       auto weights = [&](int item) {
-        const int s = item % S, g = (int)blockIdx.x + item / chunks * (int)gridDim.x, block = item % chunks * (GR_CHUNK / 32);
+        const int s = item % S, g = (int)blockIdx.x + item * (int)gridDim.x;
         mbar_expect_tx(full + s, Shape::STAGE);
-        tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, block, g * GR_ROWS, full + s, once);
+        tma_3d_once(smem_u32(smem + s * Shape::STAGE), &map_w, 0, 0, g * GR_ROWS, full + s, once);
       };
       auto rows = [&](int item) {
-        const int s = item % S, block = item % chunks * (GR_CHUNK / 32);
-        tma_3d(smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES, &map_x, 0, block, 0, full + s);
+        const int s = item % S;
+        tma_3d(smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES, &map_x, 0, 0, 0, full + s);
       };
       const int ahead = min(S, items);
       if (!early) pdl_wait();
@@ -179,31 +178,28 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     constexpr int V = (GR_ROWS * MP + 31) / 32;
     pdl_wait();                                                  // the kernel before may still read what this one overwrites
     bool ok = true;
-    float total[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) total[v] = 0.f;
     for (int i = 0; i < items; ++i) {
       const int s = i % S;
+      float total[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) total[v] = 0.f;
       if (ok) {
         ok = mbar_wait(red_full + s, (unsigned)(i / S) & 1);
         if (!ok && lane == 0) atomicExch(err, 42);
       }
       const float* slot = red + s * Shape::RED;
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int q = 0; q < GR_K / GF_SEG; ++q)
 #pragma unroll
         for (int v = 0; v < V; ++v)
           if (V * 32 == GR_ROWS * MP || lane < GR_ROWS * MP) total[v] += slot[q * (GR_ROWS * MP) + v * 32 + lane];
       __syncwarp();
       if (lane == 0) mbar_arrive(red_empty + s);
-      if (i % chunks == chunks - 1) {
-        const int n = ((int)blockIdx.x + i / chunks * (int)gridDim.x) * GR_ROWS + (lane & 15);
+      const int n = ((int)blockIdx.x + i * (int)gridDim.x) * GR_ROWS + (lane & 15);
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-          const int m = v * 2 + (lane >> 4);
-          if (m < M && n < N) C[(size_t)m * ldc + n] = total[v] + (bias ? bias[n] : 0.f);
-          total[v] = 0.f;
-        }
+      for (int v = 0; v < V; ++v) {
+        const int m = v * 2 + (lane >> 4);
+        if (m < M && n < N) C[(size_t)m * ldc + n] = total[v] + (bias ? bias[n] : 0.f);
       }
     }
     return;
@@ -214,9 +210,9 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   bool ok = true;
   unsigned parity = 0;
   const unsigned wa = smem_u32(smem + s * Shape::STAGE) + p * GR_PITCH + seg * 512;
-  const unsigned xa = smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES + mg * MT * (GR_CHUNK * 4) + seg * 512;
+  const unsigned xa = smem_u32(smem + s * Shape::STAGE) + GR_W_BYTES + mg * MT * (GR_K * 4) + seg * 512;
   for (int i = s; i < items; i += S, parity ^= 1) {
-    const int left = K - i % chunks * GR_CHUNK - seg * GF_SEG, blocks = min(4, (left + 31) / 32);        // may be <= 0
+    const int blocks = min(4, (K - seg * GF_SEG + 31) / 32);      // may be <= 0
     f32x2 acc[2][MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) acc[0][m] = acc[1][m] = 0;
@@ -231,7 +227,7 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         const ulonglong2 w0 = lds_pair(at), w1 = lds_pair(at + 8 * GR_PITCH);
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-          const ulonglong2 x = lds_pair(xa + m * (GR_CHUNK * 4) + b * 128 + c * 16);
+          const ulonglong2 x = lds_pair(xa + m * (GR_K * 4) + b * 128 + c * 16);
           acc[0][m] = fma2(w0.x, x.x, acc[0][m]);
           acc[1][m] = fma2(w1.x, x.x, acc[1][m]);
           acc[0][m] = fma2(w0.y, x.y, acc[0][m]);
@@ -246,10 +242,12 @@ gemm_f32_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       if (!ok && lane == 0) atomicExch(err, 44);
     }
     float* slot = red + s * Shape::RED + seg * (GR_ROWS * MP) + mg * (MT * GR_ROWS) + p;
+    if (seg < GR_K / GF_SEG) {
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      slot[m * GR_ROWS] = sum2(acc[0][m]);
-      slot[m * GR_ROWS + 8] = sum2(acc[1][m]);
+      for (int m = 0; m < MT; ++m) {
+        slot[m * GR_ROWS] = sum2(acc[0][m]);
+        slot[m * GR_ROWS + 8] = sum2(acc[1][m]);
+      }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(red_full + s);
@@ -493,7 +491,7 @@ static int launch_rows(const float* A, const float* W, const float* bias, float*
                        bool early, int* err, cudaStream_t s) {
   using Shape = RowsShape<MT, MG>;
   CUtensorMap mx, mw;
-  if (!make_blocks_f32(&mx, A, M, K, lda, Shape::MP, GR_CHUNK / 32, false) || !make_blocks_f32(&mw, W, N, K, ldw, GR_ROWS, 17, true)) return (int)cudaErrorInvalidValue;
+  if (!make_blocks_f32(&mx, A, M, K, lda, Shape::MP, GR_K / 32, false) || !make_blocks_f32(&mw, W, N, K, ldw, GR_ROWS, GR_K / 32 + 1, true)) return (int)cudaErrorInvalidValue;
   const cudaError_t e = cudaFuncSetAttribute(gemm_f32_rows_kernel<MT, MG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
   if (e != cudaSuccess) return (int)e;
   const int sms = device_sm_count(), groups = (N + GR_ROWS - 1) / GR_ROWS;
@@ -559,7 +557,7 @@ Q25_EXPORT int q25_gemm_f32(const float* A, const float* W, const float* bias, f
     }
     return launch_status();
   }
-  if (M <= 16 && K % 32 == 0 && lda % 32 == 0 && ldw % 32 == 0) {
+  if (M <= 16 && K <= GR_K && K % 32 == 0 && lda % 32 == 0 && ldw % 32 == 0) {
     if (M == 1) return launch_rows<1, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
     if (M == 2) return launch_rows<2, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);
     if (M <= 4) return launch_rows<4, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, early, err, s);

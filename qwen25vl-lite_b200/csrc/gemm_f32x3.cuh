@@ -3,7 +3,7 @@
 
 #include "common.cuh"
 
-// Shares of 32 k are the unit; below 256 of them a product is short enough for the FMA kernels (gemm_f32.cu).
+// Whole lines of 32 k; below 256 k the FMA kernels' shorter start counts for more (gemm_f32.cu).
 static inline bool f32x3_takes(int K) { return K >= 256 && K % 32 == 0; }
 // W aligned for TMA; A too where M <= F32X3_FEW, else `scratch` holds f32x3_scratch(M, N, K) bytes.
 #define F32X3_FEW 16

@@ -1,6 +1,7 @@
 """The 32-bit product's kernels at the edges of their tiles: a stream of the weights for up to 16 rows, 32 x 32 tiles with the
 warps side by side in K, 64 x 64 tiles, and plain loads where TMA refuses an operand.  All add in one order, so a row is the
-same bit for bit whichever of them computes it."""
+same bit for bit whichever of them computes it.  (The cases with K 512, 640, 11,008, 544, 4,096 and 384, multiples of 32 from 256 on, run on tensor
+cores: test_gemm_f32x3_gpu.py.)"""
 
 import numpy as np
 import pytest
@@ -12,6 +13,8 @@ pytestmark = pytest.mark.gpu
 CASES = [(1, 17, 4, 0), (2, 16, 36, 0), (3, 300, 512, 0), (5, 33, 516, 0), (9, 64, 1028, 12), (16, 2400, 640, 0), (4, 16, 11008, 0), (2, 40, 32, 32), (7, 50, 544, 0), (12, 5000, 96, 64),
          (17, 31, 132, 0), (64, 2048, 2052, 0), (33, 65, 4096, 4), (256, 130, 100, 0),                      # warps side by side in K
          (640, 1990, 260, 0), (700, 4100, 128, 8),                                                          # tiles of 64 x 64
+         (1, 2400, 224, 0), (2, 17, 192, 32), (3, 300, 224, 0), (4, 16, 96, 0), (7, 50, 160, 0), (8, 2500, 128, 0), (16, 2400, 224, 0),     # the stream: one and two segments
+         (33, 65, 4100, 4),                                                                                 # many rounds of warps side by side in K
          (3, 100, 257, 0), (70, 70, 64, 1)]                                                                  # plain loads
 
 
