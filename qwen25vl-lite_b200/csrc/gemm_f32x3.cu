@@ -1,4 +1,5 @@
-// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) of 32-bit operands on the tensor cores, no less precise than by 32-bit FMAs.
+// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) of 32-bit operands on the tensor cores: for operands of both signs nearer to 64 bits than by 32-bit
+// FMAs, for sums of one sign not always (below).
 //
 // A 32-bit number is the sum of three bfloat16 numbers, hi + mid + lo: hi is the number rounded, mid what hi leaves, rounded,
 // lo the rest; 8 bits of the mantissa each, so nothing is lost (below 2^-109 the rest is less than bfloat16's smallest number, and low
@@ -15,9 +16,10 @@
 //
 // The order depends on nothing but K, so a token's result is bit for bit the same whether it is computed alone, in a portion or in a
 // large batch: mma.sync and tcgen05.mma give the same bits for the same 16 k (test_gemm_f32x3_gpu.py holds them to it).
-// Error against 64 bits, relative 2-norm, random operands of both signs, by FMA (gemm_f32.cu) and here: K 256 1.49e-7 and 8.0e-8, 2,048
-// 1.66e-7 and 9.8e-8, 11,008 2.24e-7 and 1.46e-7.  Sums of one sign collect what is cut off: 6.0e-8 and 7.1e-8 at K 512, 7.0e-8 and
-// 7.3e-8 at 2,048, 1.33e-7 and 1.08e-7 at 11,008.
+// Error against 64 bits, relative 2-norm, random operands, by FMA (gemm_f32.cu) and here, at K 256 / 2,048 / 11,008: of both signs 1.49e-7 and
+// 8.0e-8, 1.66e-7 and 9.8e-8, 2.24e-7 and 1.46e-7; with exponents spread over 2^+-12 1.14e-7 and 9.0e-8, 1.35e-7 and 1.06e-7, 2.02e-7 and
+// 1.51e-7.  Sums of one sign collect what is cut off: 6.9e-8 and 7.0e-8, 6.3e-8 and 7.1e-8, 1.44e-7 and 1.15e-7 (and 5.6e-8 and 6.8e-8 at 1,024); with
+// spread exponents 9.9e-8 and 1.61e-7, 8.8e-8 and 1.56e-7, 1.46e-7 and 1.75e-7.
 // A result that is not finite (an infinite or not-a-number operand has no three parts; a part may round up to infinity), or below 2^-84
 // and not zero, is computed again by plain FMA, behind its CTA's pipeline.
 //
@@ -477,7 +479,7 @@ f3_parts_kernel(const float* __restrict__ A, uint4* __restrict__ parts, int M, i
 // Warps: 4 drain a tile of up to 64 rows, 8 a wider one (half of its columns each, which is what their registers hold); then 4
 // converters, or 8 where a chunk's MMAs leave less time (the second four take the odd chunks); a producer for W, which runs ahead
 // of the kernel before, one for A's parts, and the MMA warp.
-// Measured, 1,500 rows x 22,016 x 2,048: 586 us, 231 TFLOP/s of the product asked for (by FMA 2,988 us); a chunk takes 654 / 551 / 455 /
+// Measured, 1,500 rows x 22,016 x 2,048: 585 us with f3_parts_kernel, 231 TFLOP/s of the product asked for (by FMA 2,988 us); a chunk takes 654 / 551 / 455 /
 // 420 ns with tiles of 128 / 96 / 64 / 32 rows, which is the same 61 bytes a ns from L2 into every SM (9 TB/s) for all four: the tensor
 // pipe is busy 410 of the 654.  What the warps do between their barriers must stay short: with selects for a block's first chunk
 // (and the spills they brought), an error path in each loop and branches around the arrivals it was 814 ns.
@@ -732,15 +734,17 @@ f3_tile_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
           const float more = whole && bias ? bias[n] : 0.f;
           const size_t pitch = whole ? ldc : N;
           float* dst = (whole ? C : planes + (size_t)((c_begin + c) / F3_BLOCK_CHUNKS) * M * N) + m0 * pitch + n;
-          bool finite = true;
 #pragma unroll
           for (int j = 0; j < WIDTH; ++j, dst += pitch) {
-            const float value = acc[j] + more;
-            finite &= f3_sound(value);
-            if (m0 + j < M) *dst = value;
+            if (m0 + j < M) *dst = acc[j] + more;
             asm volatile("" : "+l"(dst));        // one address after the other: all of them at once do not fit the registers
           }
-          if (whole && !finite) *odd = 1;
+          if (whole) {                           // the planes' sums are looked at by f3_sum_kernel
+            bool sound = true;
+#pragma unroll
+            for (int j = 0; j < WIDTH; ++j) sound &= f3_sound(acc[j] + more);
+            if (!sound) *odd = 1;
+          }
         }
         __syncwarp();
 #pragma unroll
@@ -854,7 +858,7 @@ int launch_f32x3_few(const float* A, const float* W, const float* bias, float* C
 }
 
 // How f3_tile_kernel takes a product: the width of its tiles, and into how many ranges of blocks a tile is cut.  The one that ends
-// first: the chunks of the fullest SM at what a chunk takes (ns), and for a split the trip through its planes.
+// first: the chunks of the fullest SM at what a chunk takes (ns), and for a split the trip through its planes (up to 64 MB of them, half of L2).
 struct F3Plan { int bn, splits; double ns; };
 static F3Plan f3_plan(int M, int N, int K, int sms) {
   const int widths[4] = {128, 96, 64, 32}, ns[4] = {640, 540, 455, 425};
