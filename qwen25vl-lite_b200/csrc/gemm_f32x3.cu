@@ -179,7 +179,9 @@ __device__ __noinline__ void f3_again(const float* __restrict__ A, const float* 
 template <int MP, int TEAMS> struct F3Rows {     // MP: rows of x in a stage; teams of four warps
   static constexpr int TILES = MP > 8 ? 2 : 1;
   static constexpr int STAGE = F3R_W_BYTES + MP * F3R_K * 4;
-  static constexpr int STAGES = MP == 1 ? 6 : MP <= 4 ? 5 : MP == 8 ? 4 : 3;
+  // One row would have room for six, but then no CTA of a small kernel ahead (a norm) fits beside this one, which starts fetching later for it:
+  // a generation step of one request, 6 layers of the 3B sizes, 650 us, with five 637.
+  static constexpr int STAGES = MP <= 4 ? 5 : MP == 8 ? 4 : 3;
   static constexpr int VALUES = MP < 8 ? F3_BLOCK_CHUNKS : 1;    // that a team leaves of a block: its chunks', or their sum
   static constexpr int RED = F3R_K / F3_BLOCK * VALUES * F3R_FEATURES * MP;          // floats that a team leaves
   static constexpr int THREADS = (TEAMS * 4 + 2) * 32;
